@@ -5,6 +5,7 @@
 // operations, and block partials are summed in FP64; a second kernel reduces the blocks in a fixed order.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 
 #include "common.cuh"
@@ -20,84 +21,88 @@ namespace mcl {
 // Sr / Pr / count about the centre, Sr / Pr / count about the axis.
 constexpr int kExtra = 14;
 
+// At most this many blocks: each sums its share of the sites in registers (a grid stride), so the FP64 warp reduction of
+// the nine sums and the second kernel's work are paid once per block instead of once per 256 sites.
+constexpr int kExtraBlocks = 148 * 8;
+
+// Bound by instruction issue (the FP32 site terms and their FP64 sums; the director reads hit L2). Every bond is
+// taken once, from its lower end: the splay term of a bond is the same from both ends. One launch over a
+// 256 x 256 x 64 slab: see the reduction below for both kernels' times.
 template <int GEO>
 __global__ void __launch_bounds__(kThreads) k_extras(RepDesc R, const float *__restrict__ dir,
                                                      const uint8_t *__restrict__ pt, const float *__restrict__ nrm,
                                                      float d0, float d1, float d2, double *__restrict__ partials) {
-  double acc[kExtra];
-#pragma unroll
-  for (int k = 0; k < kExtra; k++) acc[k] = 0.0;
+  double splay[3] = {0.0, 0.0, 0.0}, sdiv = 0.0, spol = 0.0, rad[4] = {0.0, 0.0, 0.0, 0.0};
+  int bonds = 0, valid = 0, nrad[2] = {0, 0};
+  const float cx = (float)(R.nx / 2), cy = (float)(R.ny / 2), cz = (float)(R.nz / 2);
   const long long N = (long long)R.nx * R.ny * R.nz;
-  const long long q = (long long)blockIdx.x * kThreads + threadIdx.x;
-  if (q < N) {
+  for (long long q = (long long)blockIdx.x * kThreads + threadIdx.x; q < N; q += (long long)gridDim.x * kThreads) {
     const unsigned qq = (unsigned)q, row = qq / (unsigned)R.nx;
     const int x = (int)(qq - row * (unsigned)R.nx);
     const int z = (int)(row / (unsigned)R.ny), y = (int)(row - (unsigned)z * (unsigned)R.ny);
     Vec3 a, nb[6], s;
     float w[6];
     int sid;
-    if (gather_site_rows<GEO>(R, dir, pt, nrm, x, y, z, a, nb, w, sid, s)) {
-      // splay vector (parameter_order.cpp:158-170): every present bond, r the bond direction
+    if (!gather_site_rows<GEO>(R, dir, pt, nrm, x, y, z, a, nb, w, sid, s)) continue;
+    // splay vector (parameter_order.cpp:158-170): every present bond, r the bond direction, half from each end
 #pragma unroll
-      for (int d = 0; d < 6; d++) {
-        if (w[d] == 0.f) continue;
-        const Vec3 &b = nb[d];
-        const int ax = d >> 1;
-        const float sg = (d & 1) ? -1.f : 1.f;
-        // a.r and b.r for r = sg e_ax: the reference's sums with components 0 and +-1 are these exactly
-        const float ra = sg * (ax == 0 ? a.x : (ax == 1 ? a.y : a.z));
-        const float rb = sg * (ax == 0 ? b.x : (ax == 1 ? b.y : b.z));
-        const float ab = a.x * b.x + a.y * b.y + a.z * b.z;
-        acc[0] += 0.5 * (double)(b.x * rb - a.x * ra + a.x * ab * rb - b.x * ab * ra);
-        acc[1] += 0.5 * (double)(b.y * rb - a.y * ra + a.y * ab * rb - b.y * ab * ra);
-        acc[2] += 0.5 * (double)(b.z * rb - a.z * ra + a.z * ab * rb - b.z * ab * ra);
-        acc[3] += 1.0;
-      }
-      // divergence (parameter_order.cpp:192-210): per axis central or one-sided difference
-      double div = 0.0;
+    for (int ax = 0; ax < 3; ax++) {
+      if (w[2 * ax] == 0.f) continue;
+      const Vec3 &b = nb[2 * ax];
+      // a.r and b.r for r = e_ax: the reference's sums with components 0 and +-1 are these exactly
+      const float ra = ax == 0 ? a.x : (ax == 1 ? a.y : a.z);
+      const float rb = ax == 0 ? b.x : (ax == 1 ? b.y : b.z);
+      const float ab = a.x * b.x + a.y * b.y + a.z * b.z;
+      splay[0] += (double)(b.x * rb - a.x * ra + a.x * ab * rb - b.x * ab * ra);
+      splay[1] += (double)(b.y * rb - a.y * ra + a.y * ab * rb - b.y * ab * ra);
+      splay[2] += (double)(b.z * rb - a.z * ra + a.z * ab * rb - b.z * ab * ra);
+      bonds += 2;
+    }
+    // divergence (parameter_order.cpp:192-210): per axis central or one-sided difference
+    double div = 0.0;
 #pragma unroll
-      for (int ax = 0; ax < 3; ax++) {
-        double dd = 0.0;
-        int cnt = 0;
+    for (int ax = 0; ax < 3; ax++) {
+      const float ac = ax == 0 ? a.x : (ax == 1 ? a.y : a.z);
+      const Vec3 &bp = nb[2 * ax], &bm = nb[2 * ax + 1];
+      const float pc = ax == 0 ? bp.x : (ax == 1 ? bp.y : bp.z), mc = ax == 0 ? bm.x : (ax == 1 ? bm.y : bm.z);
+      const bool hp = w[2 * ax] != 0.f, hm = w[2 * ax + 1] != 0.f;
+      const double dd = (hm ? (double)(-(mc - ac)) : 0.0) + (hp ? (double)(pc - ac) : 0.0);
+      div += hp && hm ? 0.5 * dd : dd;  // the mean of the one or two differences
+    }
+    sdiv += div;
+    valid++;
+    // polarisation (parameter_order.cpp:135-139)
+    spol += (double)(d0 * a.x + d1 * a.y + d2 * a.z);
+    // radial orders (parameter_order.cpp:225-240)
 #pragma unroll
-        for (int sgi = 0; sgi < 2; sgi++) {  // bond 2 ax is +1, 2 ax + 1 is -1
-          const int d = 2 * ax + (sgi == 0 ? 1 : 0);
-          if (w[d] == 0.f) continue;
-          const float sg = sgi == 0 ? -1.f : 1.f;
-          const float bc = ax == 0 ? nb[d].x : (ax == 1 ? nb[d].y : nb[d].z);
-          const float ac = ax == 0 ? a.x : (ax == 1 ? a.y : a.z);
-          dd += (double)(sg * (bc - ac));
-          cnt++;
-        }
-        if (cnt) div += dd / cnt;
-      }
-      acc[4] = div;
-      acc[5] = 1.0;
-      // polarisation (parameter_order.cpp:135-139)
-      acc[6] = (double)(d0 * a.x + d1 * a.y + d2 * a.z);
-      acc[7] = 1.0;
-      // radial orders (parameter_order.cpp:225-240)
-      const float cx = (float)(R.nx / 2), cy = (float)(R.ny / 2), cz = (float)(R.nz / 2);
-#pragma unroll
-      for (int cyl = 0; cyl < 2; cyl++) {
-        const float rx = x - cx, ry = y - cy, rz = cyl ? 0.f : z - cz;
-        const float r = sqrtf(rx * rx + ry * ry + rz * rz);
-        if (r < 0.5f) continue;
-        const double c = (a.x * rx + a.y * ry + a.z * rz) / r;
-        acc[8 + 3 * cyl] = 1.5 * c * c - 0.5;
-        acc[9 + 3 * cyl] = c;
-        acc[10 + 3 * cyl] = 1.0;
-      }
+    for (int cyl = 0; cyl < 2; cyl++) {
+      const float rx = x - cx, ry = y - cy, rz = cyl ? 0.f : z - cz;
+      const float r = sqrtf(rx * rx + ry * ry + rz * rz);
+      if (r < 0.5f) continue;
+      const double c = (a.x * rx + a.y * ry + a.z * rz) / r;
+      rad[2 * cyl] += 1.5 * c * c - 0.5;
+      rad[2 * cyl + 1] += c;
+      nrad[cyl]++;
     }
   }
   __shared__ double red[kThreads / 32][kExtra];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double sums[9] = {splay[0], splay[1], splay[2], sdiv, spol, rad[0], rad[1], rad[2], rad[3]};
+  const int at[9] = {0, 1, 2, 4, 6, 8, 9, 11, 12};
 #pragma unroll
-  for (int k = 0; k < kExtra; k++) {
-    double v = acc[k];
+  for (int k = 0; k < 9; k++) {
+    double v = sums[k];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) red[warp][k] = v;
+    if (lane == 0) red[warp][at[k]] = v;
+  }
+  const int nb_ = __reduce_add_sync(0xffffffffu, bonds), nv_ = __reduce_add_sync(0xffffffffu, valid);
+  const int ns_ = __reduce_add_sync(0xffffffffu, nrad[0]), nc_ = __reduce_add_sync(0xffffffffu, nrad[1]);
+  if (lane == 0) {
+    red[warp][3] = nb_;
+    red[warp][5] = red[warp][7] = nv_;
+    red[warp][10] = ns_;
+    red[warp][13] = nc_;
   }
   __syncthreads();
   if (threadIdx.x < kExtra) {
@@ -107,12 +112,16 @@ __global__ void __launch_bounds__(kThreads) k_extras(RepDesc R, const float *__r
   }
 }
 
-__global__ void k_extras_reduce(const double *__restrict__ partials, int n_blocks, double *__restrict__ out) {
-  const int k = threadIdx.x;
-  if (k >= kExtra) return;
+// One warp per sum, its lanes over the blocks (fixed order).
+__global__ void __launch_bounds__(32 * kExtra) k_extras_reduce(const double *__restrict__ partials, int n_blocks,
+                                                               double *__restrict__ out) {
+  const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double v = 0.0;
-  for (int b = 0; b < n_blocks; b++) v += partials[(long long)b * kExtra + k];
-  out[k] = v;
+#pragma unroll 8
+  for (int b = lane; b < n_blocks; b += 32) v += partials[(long long)b * kExtra + k];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane == 0) out[k] = v;
 }
 
 // Local order parameter of every site (src/parameter_order.cpp:75-127): Q over the site and its present
@@ -175,11 +184,9 @@ extern "C" int mcl_measure_extras(mcl_engine *e, int replica, const double direc
   if (!e->geometry_set) return fail(MCL_ERR_STATE, "custom geometry: call mcl_set_geometry first");
   const RepDesc &D = e->desc[replica];
   const long long N = (long long)D.nx * D.ny * D.nz;
-  const int n_blocks = (int)((N + kThreads - 1) / kThreads);
-  if (!e->d_xpart) {  // first call: scratch for the largest replica
-    const long long most = (e->max_sites + kThreads - 1) / kThreads;
-    CKX(cudaMalloc(&e->d_xpart, (size_t)(most * kExtra + kExtra) * sizeof(double)));
-  }
+  const int n_blocks = (int)std::min<long long>((N + kThreads - 1) / kThreads, kExtraBlocks);
+  if (!e->d_xpart)  // first call: scratch for any replica
+    CKX(cudaMalloc(&e->d_xpart, (size_t)(kExtraBlocks * kExtra + kExtra) * sizeof(double)));
   double *partials = e->d_xpart, *sums = e->d_xpart + (size_t)n_blocks * kExtra;
   const LaunchCtx c = e->ctx();
   const float d0 = (float)director[0], d1 = (float)director[1], d2 = (float)director[2];
@@ -194,7 +201,7 @@ extern "C" int mcl_measure_extras(mcl_engine *e, int replica, const double direc
       k_extras<GEO_PT><<<n_blocks, kThreads, 0, c.stream>>>(D, c.dir, c.pt, c.nrm, d0, d1, d2, partials);
   }
   CKX(cudaGetLastError());
-  k_extras_reduce<<<1, 32, 0, c.stream>>>(partials, n_blocks, sums);
+  k_extras_reduce<<<1, 32 * kExtra, 0, c.stream>>>(partials, n_blocks, sums);
   CKX(cudaGetLastError());
   e->launches += 2;
   double v[kExtra];
