@@ -562,7 +562,22 @@ int mcl_get_sweep_counter(mcl_engine *e, unsigned long long *sweep) {
 
 static int sweeps_run(mcl_engine *e, int n, int measure);
 
+static int sweeps_all(mcl_engine *e, int n, int measure);
+
 int mcl_sweeps(mcl_engine *e, int n, int measure) {
+  const int first = e ? e->series_len : 0;
+  const int rc = sweeps_all(e, n, measure);
+  if (!e || !measure || e->series_len == first) return rc;
+  const long long rows = e->series_len - first;  // also after an error: the sweeps that were queued have records
+  const cudaError_t ce = launch_series_eigen(e->stream, e->d_series, (long long)first * e->n_rep, rows * e->n_rep);
+  e->launches++;
+  if (rc) return rc;
+  CK(ce);
+  return MCL_OK;
+}
+
+// The sweeps of mcl_sweeps; the new records' S and director are left to the caller.
+static int sweeps_all(mcl_engine *e, int n, int measure) {
   if (!e) return fail(MCL_ERR_ARG, "null engine");
   if (n < 0) return fail(MCL_ERR_ARG, "negative sweep count");
   if (e->zslab) return fail(MCL_ERR_STATE, "mcl_sweeps: a z-slab engine sweeps through the mcl_zslab_* calls");
@@ -757,7 +772,7 @@ int mcl_sweeps_io(mcl_engine *e, int n, const float *T, mcl_observables *out) {
       e->launches++;
     }
     const int first = e->series_len;
-    if ((rc = mcl_sweeps(e, n, 1))) return rc;
+    if ((rc = sweeps_all(e, n, 1))) return rc;
     e->io_inflight = true;
     CK(launch_io_out(e->stream, e->d_series, first, nullptr, n, e->n_rep, (ObsRecord *)(dio + rec_off),
                      fused_error_word(e), e->d_lerr, (unsigned *)dio));
@@ -1087,7 +1102,11 @@ int mcl_zslab_finalize(mcl_engine *e, const double *d_sums, int measure) {
   int rc;
   if (measure && (rc = ensure_series(e, e->series_len + 1))) return rc;
   if ((rc = fused_finalize_global(e, d_sums, measure ? 1 : 0))) return rc;
-  if (measure) e->series_len++;
+  if (measure) {
+    CK(launch_series_eigen(e->stream, e->d_series, (long long)e->series_len * e->n_rep, e->n_rep));
+    e->launches++;
+    e->series_len++;
+  }
   return MCL_OK;
 }
 

@@ -116,10 +116,11 @@ __global__ void __launch_bounds__(kThreads) k_observe(ModelDev m, const RepDesc 
 }
 
 // ------------------------------------------------------------------------------------------------------------
-// One block per replica: deterministic reduction of the replica's partials, S and director by Jacobi, ang_var
-// adaptation (src/evolve.cpp:211-220; skipped when adapt = 0), optional series record, reset of the acceptance
-// counter. The last
-// block to finish advances the global sweep counter and the series length. measure: 0 none, 1 append to the
+// One block per replica: deterministic reduction of the replica's partials, ang_var adaptation
+// (src/evolve.cpp:211-220; skipped when adapt = 0), optional series record, reset of the acceptance counter. A
+// series record is left without S and director, which nothing in the sweep loop reads: the serial FP64 Jacobi solve
+// (3-5 us) would stand between two sweeps, so k_series_eigen solves all records of a call at once, one per thread. A
+// probe record is solved here. The last block to finish advances the global sweep counter and the series length. measure: 0 none, 1 append to the
 // series, 2 probe (record the current state into series[rep]; no adaptation, counters untouched). gsums (z-slab
 // processes): the observables and accepted rotations already summed over all processes (kZslabSums per replica)
 // replace the local partials and the local acceptance counter.
@@ -142,6 +143,8 @@ __global__ void __launch_bounds__(kThreads) k_finalize(const RepDesc *__restrict
     double acc[kPartials];
 #pragma unroll
     for (int k = 0; k < kPartials; k++) acc[k] = 0.0;
+    // unrolled: the loads of several items are in flight together (the sums' order does not change)
+#pragma unroll 4
     for (int b = obs_first[rep] + threadIdx.x; b < obs_first[rep + 1]; b += kThreads)
 #pragma unroll
       for (int k = 0; k < kPartials; k++) acc[k] += partials[(long long)b * kPartials + k];
@@ -185,12 +188,8 @@ __global__ void __launch_bounds__(kThreads) k_finalize(const RepDesc *__restrict
       ObsRecord o;
       o.energy = tot[0] / nv;
       for (int k = 0; k < 6; k++) o.q[k] = tot[1 + k] / nv;
-      double vec[3];
-      o.S = largest_eigen3(o.q, vec);
-      for (int k = 0; k < 3; k++) {
-        o.director[k] = vec[k];
-        o.nsum[k] = tot[7 + k];
-      }
+      if (probe) o.S = largest_eigen3(o.q, o.director);
+      for (int k = 0; k < 3; k++) o.nsum[k] = tot[7 + k];
       o.n_valid = nv;
       o.acceptance = a;
       o.ang_var = av;
@@ -344,6 +343,26 @@ cudaError_t launch_observe(const LaunchCtx &c, int geo, const BlockTable &sites,
   return cudaGetLastError();
 }
 
+// S and director of `count` consecutive series records, one thread each.
+__device__ __forceinline__ void solve_record(ObsRecord *r) {
+  double q[6], vec[3];
+#pragma unroll
+  for (int k = 0; k < 6; k++) q[k] = r->q[k];
+  r->S = largest_eigen3(q, vec);
+#pragma unroll
+  for (int k = 0; k < 3; k++) r->director[k] = vec[k];
+}
+
+__global__ void __launch_bounds__(32) k_series_eigen(ObsRecord *__restrict__ series, long long first, long long count) {
+  const long long i = (long long)blockIdx.x * 32 + threadIdx.x;
+  if (i < count) solve_record(series + first + i);
+}
+
+cudaError_t launch_series_eigen(cudaStream_t stream, ObsRecord *series, long long first, long long count) {
+  if (count > 0) k_series_eigen<<<(unsigned)((count + 31) / 32), 32, 0, stream>>>(series, first, count);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_finalize(const LaunchCtx &c, const BlockTable &sites, const double *partials, int measure,
                             ObsRecord *series, int *series_len, unsigned int *done_ctr, const double *gsums) {
   k_finalize<<<c.n_replicas, kThreads, 0, c.stream>>>(c.reps, c.state, sites.first, partials, measure, series,
@@ -422,17 +441,25 @@ __global__ void k_io_in(RepState *__restrict__ st, const float *__restrict__ hos
 }
 
 // series_len non-null (a captured graph, whose arguments are fixed): the rows are the newest n_rows, and first_row is
-// ignored.
-__global__ void k_io_out(const ObsRecord *__restrict__ series, long long first_row, const int *__restrict__ series_len,
-                         int n_rows, int n_rep, ObsRecord *__restrict__ host_rec, const unsigned *__restrict__ err0,
-                         const unsigned *__restrict__ err1, unsigned *__restrict__ host_words) {
+// ignored. Every block solves its own records (S, director), then copies them out.
+constexpr int kIoRecords = 32;  // records per block, one solver thread each
+__global__ void __launch_bounds__(128) k_io_out(ObsRecord *__restrict__ series, long long first_row,
+                                                const int *__restrict__ series_len, int n_rows, int n_rep,
+                                                ObsRecord *__restrict__ host_rec, const unsigned *__restrict__ err0,
+                                                const unsigned *__restrict__ err1,
+                                                unsigned *__restrict__ host_words) {
   static_assert(sizeof(ObsRecord) % 8 == 0, "records move as 8-byte words");
   if (series_len) first_row = max(0, *series_len - n_rows);
-  const long long words = (long long)n_rows * n_rep * (long long)(sizeof(ObsRecord) / 8);
-  const unsigned long long *src = reinterpret_cast<const unsigned long long *>(series + first_row * n_rep);
-  unsigned long long *dst = reinterpret_cast<unsigned long long *>(host_rec);
-  for (long long i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
-  if (threadIdx.x == 0) {
+  const long long first = (long long)blockIdx.x * kIoRecords, all = (long long)n_rows * n_rep;
+  const int mine = (int)min((long long)kIoRecords, all - first);
+  ObsRecord *rec = series + first_row * n_rep + first;
+  if ((int)threadIdx.x < mine) solve_record(rec + threadIdx.x);
+  __syncthreads();
+  const unsigned long long *src = reinterpret_cast<const unsigned long long *>(rec);
+  unsigned long long *dst = reinterpret_cast<unsigned long long *>(host_rec + first);
+  const int words = mine * (int)(sizeof(ObsRecord) / 8);
+  for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
     host_words[0] = err0 ? *err0 : 0u;
     host_words[1] = err1 ? *err1 : 0u;
   }
@@ -443,11 +470,12 @@ cudaError_t launch_io_in(cudaStream_t stream, RepState *st, const float *host_T,
   return cudaGetLastError();
 }
 
-cudaError_t launch_io_out(cudaStream_t stream, const ObsRecord *series, long long first_row, const int *series_len,
+cudaError_t launch_io_out(cudaStream_t stream, ObsRecord *series, long long first_row, const int *series_len,
                           int n_rows, int n_rep, ObsRecord *host_rec, const unsigned *err0, const unsigned *err1,
                           unsigned *host_words) {
-  k_io_out<<<1, kThreads, 0, stream>>>(series, first_row, series_len, n_rows, n_rep, host_rec, err0, err1,
-                                       host_words);
+  const long long blocks = ((long long)n_rows * n_rep + kIoRecords - 1) / kIoRecords;
+  k_io_out<<<(unsigned)blocks, 128, 0, stream>>>(series, first_row, series_len, n_rows, n_rep, host_rec, err0, err1,
+                                                 host_words);
   return cudaGetLastError();
 }
 

@@ -45,15 +45,18 @@ cudaError_t launch_observe(const LaunchCtx &c, int geo, const BlockTable &sites,
 cudaError_t launch_zslab_planes(const LaunchCtx &c, float *dir, float *lo, float *hi, int pack);
 // mcl_sweeps_io's step input (temperatures from mapped host memory into the replicas' state) and output (series rows
 // first_row .. first_row + n_rows - 1, or with series_len the newest n_rows, and the error words, null for absent
-// ones, into mapped host memory).
+// ones, into mapped host memory; it solves the records for S and director first).
 cudaError_t launch_io_in(cudaStream_t stream, RepState *st, const float *host_T, int n_rep);
-cudaError_t launch_io_out(cudaStream_t stream, const ObsRecord *series, long long first_row, const int *series_len,
+cudaError_t launch_io_out(cudaStream_t stream, ObsRecord *series, long long first_row, const int *series_len,
                           int n_rows, int n_rep, ObsRecord *host_rec, const unsigned *err0, const unsigned *err1,
                           unsigned *host_words);
 // Per-replica sums of the partials over a block table and the accepted rotations (kZslabSums doubles each).
 cudaError_t launch_item_sums(const LaunchCtx &c, const BlockTable &items, const double *partials, int measure,
                              double *out);
-// Per-replica reduction of the partials, S by Jacobi, ang_var adaptation, series record, counter advance; with
+// S and director (Jacobi) of `count` series records from record `first` on: the part of a record that k_finalize
+// leaves to the end of a call.
+cudaError_t launch_series_eigen(cudaStream_t stream, ObsRecord *series, long long first, long long count);
+// Per-replica reduction of the partials, ang_var adaptation, series record, counter advance; with
 // gsums, from sums already reduced over z-slab processes instead of the local partials and acceptance counter.
 cudaError_t launch_finalize(const LaunchCtx &c, const BlockTable &sites, const double *partials, int measure,
                             ObsRecord *series, int *series_len, unsigned int *done_ctr,
