@@ -211,6 +211,10 @@ int mcl_local_order(mcl_engine *e, int replica, float *S);
  *   2: two in-place colour passes per sweep, 64 x 16 sites, 256 threads, 3 CTAs per SM;
  *   3: colour passes, 64 x 16 sites, 256 threads, 2 CTAs per SM (flip models: two trials per site);
  *   4: colour passes, 32 x 16 sites, 128 threads, 5 CTAs per SM (narrow lattices waste less of a tile).
+ * Without a plan asked for (mcl_set_plan, mcl_autotune), an engine whose replicas are small sweeps them in shared
+ * memory instead, one cluster of CTAs per replica and all sweeps of a call in one launch; mcl_get_plan then names the
+ * tile plan it would use otherwise. mcl_autotune times that kernel too and, where it is the fastest, keeps it (the
+ * plan fields of *out are then the default plan's).
  * The fused configurations need a second director buffer, allocated while one of them is selected and freed when a
  * colour-pass configuration is selected again. Every configuration gives bit-identical directors. Candidate plans:
  * per configuration the heuristic segment length, its double, its half and the whole depth; lattices that give

@@ -610,11 +610,41 @@ int mcl_set_proposal_mix(mcl_engine *e, int period) {
   return MCL_OK;
 }
 
+// The next pair of profiling events, around `sweeps` sweeps.
+static int profile_events(mcl_engine *e, int sweeps, cudaEvent_t *ev0, cudaEvent_t *ev1) {
+  while (e->ev_pool.size() < e->ev_used + 2) {
+    cudaEvent_t ev;
+    CK(cudaEventCreate(&ev));
+    e->ev_pool.push_back(ev);
+  }
+  e->ev_sweeps.resize(e->ev_used / 2 + 1);
+  e->ev_sweeps[e->ev_used / 2] = sweeps;
+  *ev0 = e->ev_pool[e->ev_used];
+  *ev1 = e->ev_pool[e->ev_used + 1];
+  e->ev_used += 2;
+  return MCL_OK;
+}
+
 static int sweeps_run(mcl_engine *e, int n, int measure) {
   int rc;
   if (measure && (rc = ensure_series(e, e->series_len + n))) return rc;
   const bool use_fused = e->fused && !e->record_dec && !e->d_mlp;
   if (use_fused && (rc = refresh_ghosts(e))) return rc;
+  if (use_fused && fused_resident(e)) {
+    // one launch for up to kResidentSweeps sweeps (bounded, so that a long call leaves the device now and then)
+    constexpr int kResidentSweeps = 1024;
+    while (n > 0) {
+      const int run = std::min(n, kResidentSweeps);
+      cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+      if (e->profile && (rc = profile_events(e, run, &ev0, &ev1))) return rc;
+      if (ev0) CK(cudaEventRecord(ev0, e->stream));
+      if ((rc = fused_resident_sweeps(e, run, measure != 0))) return rc;
+      if (ev1) CK(cudaEventRecord(ev1, e->stream));
+      if (measure) e->series_len += run;
+      n -= run;
+    }
+    return MCL_OK;
+  }
   const int per_graph = use_fused ? graph_sweeps(e) : 2;
   if (use_fused && e->use_graphs && !e->profile && n >= per_graph) {
     const int m = measure ? 1 : 0;
@@ -634,16 +664,7 @@ static int sweeps_run(mcl_engine *e, int n, int measure) {
   }
   for (int s = 0; s < n; s++) {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    if (e->profile) {
-      while (e->ev_pool.size() < e->ev_used + 2) {
-        cudaEvent_t ev;
-        CK(cudaEventCreate(&ev));
-        e->ev_pool.push_back(ev);
-      }
-      ev0 = e->ev_pool[e->ev_used];
-      ev1 = e->ev_pool[e->ev_used + 1];
-      e->ev_used += 2;
-    }
+    if (e->profile && (rc = profile_events(e, 1, &ev0, &ev1))) return rc;
     if (use_fused) {
       if ((rc = fused_sweep(e, measure != 0, ev0, ev1))) return rc;
     } else {
@@ -730,6 +751,7 @@ int mcl_sweeps_io(mcl_engine *e, int n, const float *T, mcl_observables *out) {
   // the sweep's kernels, output kernel reading the newest record), captured again when a buffer it uses moves.
   const bool use_fused = e->fused && !e->record_dec && !e->d_mlp;
   if (T && n == 1 && use_fused && e->use_graphs && !e->profile && fused_is_pass_plan(e)) {
+    const bool resident = fused_resident(e);
     if ((rc = ensure_series(e, e->series_len + 1))) return rc;
     if ((rc = refresh_ghosts(e))) return rc;
     if (!e->graph_io || e->graph_io_series != (const void *)e->d_series || e->graph_io_stage != e->d_io) {
@@ -738,8 +760,9 @@ int mcl_sweeps_io(mcl_engine *e, int n, const float *T, mcl_observables *out) {
       cudaGraph_t g = nullptr;
       CK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
       const long long l0 = e->launches;
+      rc = MCL_OK;
       cudaError_t ce = launch_io_in(e->stream, e->d_state, (const float *)(dio + t_off), e->n_rep);
-      rc = ce == cudaSuccess ? fused_sweep(e, true, nullptr, nullptr) : MCL_OK;
+      if (ce == cudaSuccess) rc = resident ? fused_resident_sweeps(e, 1, true) : fused_sweep(e, true, nullptr, nullptr);
       if (ce == cudaSuccess && !rc)
         ce = launch_io_out(e->stream, e->d_series, 0, e->d_series_len, 1, e->n_rep, (ObsRecord *)(dio + rec_off),
                            fused_error_word(e), e->d_lerr, (unsigned *)dio);
@@ -762,7 +785,7 @@ int mcl_sweeps_io(mcl_engine *e, int n, const float *T, mcl_observables *out) {
     memcpy(hT, T, (size_t)e->n_rep * sizeof(float));
     e->io_inflight = true;
     CK(cudaGraphLaunch(e->graph_io, e->stream));
-    e->launches += 2 + fused_launches_per_sweep(e);
+    e->launches += 2 + (resident ? 1 : fused_launches_per_sweep(e));
     e->series_len++;
   } else {
     if (T) {
@@ -806,7 +829,7 @@ int mcl_profile_read(mcl_engine *e, double *ms, long long *sweeps, long long *la
     float t = 0;
     CK(cudaEventElapsedTime(&t, e->ev_pool[k], e->ev_pool[k + 1]));
     e->prof_ms += t;
-    e->prof_sweeps++;
+    e->prof_sweeps += e->ev_sweeps[k / 2];
   }
   e->ev_used = 0;
   if (ms) *ms = e->prof_ms;
@@ -974,8 +997,14 @@ int mcl_autotune(mcl_engine *e, int trial_sweeps, mcl_tuning *out) {
   if (std::find(cand.begin(), cand.end(), std::make_pair(cfg0, seg0)) == cand.end()) cand.push_back({cfg0, seg0});
   double best = 1e300, t_default = 0;
   std::pair<int, int> pick{cfg0, seg0};
+  const bool asked0 = fused_release_plan(e);
+  bool resident = fused_resident(e);  // where the engine would choose the resident kernel, it is the first candidate
+  const bool default_resident = resident && !asked0;
+  const size_t n_cand = cand.size() + (resident ? 1 : 0);
+  bool pick_resident = false;
+  if (resident) cand.insert(cand.begin(), {cfg0, seg0});
   for (const auto &c : cand) {
-    if ((rc = fused_set_plan(e, c.first, c.second))) return done(rc);
+    if (!resident && (rc = fused_set_plan(e, c.first, c.second))) return done(rc);
     if ((rc = mcl_sweeps(e, 1, 1))) return done(rc);  // warm-up
     CKT(cudaEventRecord(ev0, e->stream));
     if ((rc = mcl_sweeps(e, trial_sweeps, 1))) return done(rc);
@@ -984,15 +1013,18 @@ int mcl_autotune(mcl_engine *e, int trial_sweeps, mcl_tuning *out) {
     float ms = 0.f;
     CKT(cudaEventElapsedTime(&ms, ev0, ev1));
     const double per = ms / trial_sweeps;
-    if (c.first == cfg0 && c.second == seg0) t_default = per;
+    if (default_resident ? resident : (!resident && c.first == cfg0 && c.second == seg0)) t_default = per;
     if (per < best) {
       best = per;
       pick = c;
+      pick_resident = resident;
     }
+    resident = false;
     if ((rc = restore())) return done(rc);
     if ((rc = fused_check_error(e))) return done(rc);
   }
   if ((rc = fused_set_plan(e, pick.first, pick.second))) return done(rc);
+  if (pick_resident) fused_release_plan(e);
   if (out) {
     int ty = 0, seg = 0, items = 0;
     fused_get_cfg(e, nullptr, &ty, &seg, &items);
@@ -1001,7 +1033,7 @@ int mcl_autotune(mcl_engine *e, int trial_sweeps, mcl_tuning *out) {
     out->threads_per_cta = fused_threads(pick.first);
     out->planes_per_segment = seg;
     out->work_items = items;
-    out->candidates = (int)cand.size();
+    out->candidates = (int)n_cand;
     out->ms_per_sweep = best;
     out->ms_default = t_default;
   }

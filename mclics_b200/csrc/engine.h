@@ -67,6 +67,7 @@ struct mcl_engine {
   bool zslab = false;  // replica 0 is a z-slab of a larger lattice (mcl_zslab_init): pass-level API only
   std::vector<cudaEvent_t> ev_pool;  // pairs (start, stop) of timed sweeps
   size_t ev_used = 0;
+  std::vector<int> ev_sweeps;  // sweeps between the events of each pair
   double prof_ms = 0;          // time of already-read event pairs
   long long prof_sweeps = 0;
   long long launches = 0;      // kernels launched by this engine

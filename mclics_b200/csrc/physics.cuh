@@ -152,14 +152,17 @@ __device__ __forceinline__ L ll_acc(const V3<L> &x, const V3<L> &y, const L &w, 
   return D == 0 ? mul_(mul_(w, b), b) : fma_(mul_(w, b), b, s);
 }
 template <bool PXY, typename L>
-__device__ __forceinline__ L ll_sum(const ModelDev &m, const V3<L> &x, const V3<L> (&nb)[6], const L (&w)[6]) {
+__device__ __forceinline__ L ll_sum_raw(const V3<L> &x, const V3<L> (&nb)[6], const L (&w)[6]) {
   L s = ll_acc<PXY, 0>(x, nb[0], w[0], w[0]);
   s = ll_acc<PXY, 1>(x, nb[1], w[1], s);
   s = ll_acc<PXY, 2>(x, nb[2], w[2], s);
   s = ll_acc<PXY, 3>(x, nb[3], w[3], s);
   s = ll_acc<PXY, 4>(x, nb[4], w[4], s);
-  s = ll_acc<PXY, 5>(x, nb[5], w[5], s);
-  return mul_(splat<L>(-1.5f * m.A), s);
+  return ll_acc<PXY, 5>(x, nb[5], w[5], s);
+}
+template <bool PXY, typename L>
+__device__ __forceinline__ L ll_sum(const ModelDev &m, const V3<L> &x, const V3<L> (&nb)[6], const L (&w)[6]) {
+  return mul_(splat<L>(-1.5f * m.A), ll_sum_raw<PXY>(x, nb, w));
 }
 
 // GHRL without the chiral term as sums over the site's bonds. With a_i = n.r, a_j = n_j.r, b = n.n_j, the pair
@@ -434,7 +437,7 @@ __device__ __forceinline__ V3<L> sel3(LB<L> c, const V3<L> &a, const V3<L> &b) {
 // FIELD (field term), SINGLE = false (the caller knows the site has no single-site term: no surface, no field;
 // the energies are then the bond sums themselves, which is what adding the zero single term gives, up to the sign
 // of a zero). Every combination rounds like the general one on the inputs it applies to.
-template <int POT, bool FLIP, bool PXY, bool CHIRAL, bool FIELD, typename L, bool SINGLE = true>
+template <int POT, bool FLIP, bool PXY, bool CHIRAL, bool FIELD, typename L, bool SINGLE = true, bool ENERGY = true>
 __device__ __forceinline__ SiteResultT<L> site_update(const ModelDev &m, const V3<L> &n, const V3<L> (&nb)[6],
                                                       const L (&w)[6], int sid, const Vec3 &s, float elecE,
                                                       const LaneDraw<L> &d, float av, float T, float invT) {
@@ -446,7 +449,14 @@ __device__ __forceinline__ SiteResultT<L> site_update(const ModelDev &m, const V
   const L s_new = SINGLE ? single_energy<FIELD>(m, nn, sid, s, elecE) : splat<L>(0.f);
   const L e_old = SINGLE ? add_(b_old, s_old) : b_old, e_new = SINGLE ? add_(b_new, s_new) : b_new;
   SiteResultT<L> r;
-  r.rot = metropolis(d.u3, sub_(e_new, e_old), invT, T);
+  L dE;
+  if (POT == POT_LL && !SINGLE && !ENERGY) {
+    const L c = splat<L>(-1.5f * m.A);
+    dE = fma_(c, ll_sum_raw<PXY>(nn, nb, w), neg_(mul_(c, ll_sum_raw<PXY>(n, nb, w))));
+  } else {
+    dE = sub_(e_new, e_old);
+  }
+  r.rot = metropolis(d.u3, dE, invT, T);
   r.n = sel3<L>(r.rot, nn, n);
   r.bond = sel_(r.rot, b_new, b_old);
   r.single = SINGLE ? sel_(r.rot, s_new, s_old) : splat<L>(0.f);

@@ -5,10 +5,14 @@
 
 #include <algorithm>
 #include <cmath>
+#include <functional>
+#include <map>
+#include <mutex>
 #include <vector>
 
 #include "fused.h"
 #include "sweep_pass.cuh"
+#include "sweep_resident.cuh"
 
 namespace mcl {
 
@@ -32,6 +36,9 @@ struct FusedPlan {
   size_t smem = 0;
   long long timeout_ns = 2000000000ll;
   int skip_first_load = 0;
+  bool asked = false;          // a plan was asked for (mcl_set_plan, the autotuner, MCL_FUSED_CFG)
+  int res_cluster = 0;         // CTAs per replica of the resident kernel (0: it is not used)
+  size_t res_smem = 0;
 };
 
 // ---- host side ----------------------------------------------------------------------------------------------
@@ -119,6 +126,7 @@ static int choose_cfg(const mcl_engine *e) {
 
 static int prepare_kernel(mcl_engine *e, FusedPlan *P);
 static void free_plan(FusedPlan *P);
+static void resident_choose(const mcl_engine *e, FusedPlan *P);
 
 // The fused plans read one director buffer and write the other; the colour passes and the learned passes update
 // one buffer in place. The second buffer (211 MB for a 256^3 lattice) therefore exists only while a fused plan is
@@ -199,9 +207,12 @@ int fused_create(mcl_engine *e) {
   FusedPlan *P = new FusedPlan();
   e->fused = P;
   P->cfg = choose_cfg(e);
+  P->asked = getenv("MCL_FUSED_CFG") != nullptr;
   CKF(cudaMalloc(&P->d_err, sizeof(unsigned int)));
   CKF(cudaMemset(P->d_err, 0, sizeof(unsigned int)));
-  return build_items(e, P);
+  const int rc = build_items(e, P);
+  if (rc == MCL_OK) resident_choose(e, P);
+  return rc;
 }
 
 // Selects a plan and rebuilds the work items, tensor maps and buffers for it; if that fails (an allocation), the
@@ -223,6 +234,7 @@ int fused_set_cfg(mcl_engine *e, int cfg) {
   if (!e->fused) return fail(MCL_ERR_STATE, "this engine does not use the fused tiled sweep");
   if (cfg < 0 || cfg >= kNumCfgs) return fail(MCL_ERR_ARG, "tile configuration %d outside 0..%d", cfg, kNumCfgs - 1);
   CKF(cudaStreamSynchronize(e->stream));
+  e->fused->asked = true;
   return apply_plan(e, cfg, e->fused->seg_override);
 }
 
@@ -232,6 +244,7 @@ int fused_set_plan(mcl_engine *e, int cfg, int seg) {
   if (kCfgs[cfg].kind == 0 && e->zslab)
     return fail(MCL_ERR_STATE, "a z-slab engine runs the colour passes (tile configurations 2-%d)", kNumCfgs - 1);
   CKF(cudaStreamSynchronize(e->stream));
+  e->fused->asked = true;
   return apply_plan(e, cfg, std::max(0, seg));
 }
 
@@ -319,6 +332,139 @@ void fused_destroy(mcl_engine *e) {
   cudaFree(P->d_err);
   delete P;
   e->fused = nullptr;
+}
+
+// ---- the resident kernel -------------------------------------------------------------------------------------
+static ResidentLaunch resident_desc(const mcl_engine *e, int cluster, size_t smem) {
+  ResidentLaunch l{};
+  l.geo = e->geo;
+  l.clusters = e->n_rep;
+  l.cluster_size = cluster;
+  l.flip = e->model.flip != 0 || e->model.potential == POT_PEAR;
+  l.pxy = true;
+  for (const auto &D : e->desc) l.pxy = l.pxy && D.periodic[0] && D.periodic[1];
+  l.chiral = e->model.potential == POT_GHRL && e->model.sigma != 0.f;
+  l.field = e->model.field_on != 0;
+  l.smem = smem;
+  l.stream = e->stream;
+  return l;
+}
+
+static cudaError_t resident_dispatch(const mcl_engine *e, const ResidentArgs &a, const ResidentLaunch &l) {
+  if (e->model.potential == POT_GHRL) return launch_resident_ghrl(e->model, a, l);
+  if (e->model.potential == POT_PEAR) return launch_resident_pear(e->model, a, l);
+  return launch_resident_ll(e->model, a, l);
+}
+
+// Clusters of C CTAs that run at once on the engine's device: a property of the device, since every resident kernel
+// takes a whole SM per CTA (512 threads of 128 registers). The query takes about a millisecond, so its answers are kept.
+static int clusters_that_fit(const mcl_engine *e, int C) {
+  static std::mutex mu;
+  static std::map<std::pair<int, int>, int> known;
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = known.find({e->device, C});
+  if (it != known.end()) return it->second;
+  int fit = 0;
+  ResidentLaunch l = resident_desc(e, C, kResMaxSmem);
+  l.max_clusters = &fit;
+  if (resident_dispatch(e, ResidentArgs{}, l) != cudaSuccess) {
+    cudaGetLastError();
+    fit = 0;
+  }
+  known[{e->device, C}] = fit;
+  return fit;
+}
+
+// CTAs per replica of the resident kernel, or 0 where the colour passes are faster or a replica does not fit.
+//
+// Measured per sweep on one B200 (us, unmeasured / measured sweeps in long calls; colour passes on their best plan with
+// graph replay):
+//                     resident, C = 4     C = 8          C = 16         colour passes
+//   LL 16^3           3.6 / 4.5           3.2 / 4.0      3.5 / 4.2      14.4 / 16.5
+//   LL 32^3           12.9 / 14.3         7.8 / 8.5      6.7 / 6.9      14.4 / 16.5
+//   LL 48^3           does not fit        does not fit   12.8 / 13.6    14.4 / 18.6
+//   GHRL 32^3         16.4 / 17.6         9.5 / 10.1     7.6 / 7.8      14.4 / 16.5
+//   chiral 32^3       20.2 / 21.7         11.5 / 12.2    8.6 / 8.8      14.4 / 18.4
+//   pear 48 x 48 x 24 41 / 45             23.6 / 25.4    18.0 / 19.7    24.7 / 26.9
+//   LL 32 x 32^3      13.2 / 16.8         23.3 / 27.9    32.4 / 37.2    26.8 / 30.8
+//   LL 64 x 24^3      15.1 / 18.4         25.4 / 30.2    44.2 / 74.9    37.5 / 41.0
+//   LL 128 x 16^3     14.4 / 20.0         28.0 / 40.5    62.6 / 86.9    30.8 / 33.0
+// A colour costs a chain of one task or the issue of the tasks of a full CTA, `round` us per 512, and a cluster barrier
+// that grows with C; replicas beyond the clusters that fit the device (33, 15 and 7) wait for a free one. The colour
+// passes cost three launches (14.4 us) or the same rounds over all SMs.
+static void resident_choose(const mcl_engine *e, FusedPlan *P) {
+  P->res_cluster = 0;
+  const bool flip = e->model.flip != 0 || e->model.potential == POT_PEAR;
+  const bool chiral = e->model.potential == POT_GHRL && e->model.sigma != 0.f;
+  const double round = (flip ? (e->model.potential == POT_LL ? 2.2 : 3.3) : chiral ? 2.4 : e->model.potential == POT_GHRL ? 1.9 : 1.45);
+  int min_nz = 1 << 30, sms = 148;
+  double all_tasks = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
+  for (const auto &D : e->desc) {
+    min_nz = std::min(min_nz, D.nz);
+    all_tasks += (double)D.nz * D.ny * res_pairs(D.nx);
+  }
+  ResidentLaunch limits = resident_desc(e, 1, 0);
+  limits.prepare = true;
+  if (resident_dispatch(e, ResidentArgs{}, limits) != cudaSuccess) {
+    cudaGetLastError();  // this combination of options has no kernel
+    return;
+  }
+  double best = std::max(flip ? 22.0 : 14.4, 6.0 + 2.0 * round * 1.1 * all_tasks / ((double)kResThreads * sms));
+  for (int C = 1; C <= kResMaxC && C <= min_nz; C *= 2) {
+    size_t smem = 0;
+    for (const auto &D : e->desc)
+      smem = std::max(smem, kResHead + ((size_t)(D.nz + C - 1) / C + 2) * res_plane(D.nx, D.ny) * sizeof(float));
+    if (smem > kResMaxSmem) continue;
+    const int fit = clusters_that_fit(e, C);
+    if (fit < 1) continue;
+    // replicas in order onto the cluster that is free first
+    std::vector<double> busy((size_t)std::min(fit, e->n_rep), 0.0);
+    std::make_heap(busy.begin(), busy.end(), std::greater<double>());
+    double cost = 0;
+    for (const auto &D : e->desc) {
+      const double tasks = std::ceil((double)D.nz / C) * D.ny * res_pairs(D.nx);
+      std::pop_heap(busy.begin(), busy.end(), std::greater<double>());
+      busy.back() += 2.0 * (std::max(0.8, round * tasks / kResThreads) + 0.4 + 0.08 * C);
+      cost = std::max(cost, busy.back());
+      std::push_heap(busy.begin(), busy.end(), std::greater<double>());
+    }
+    if (cost < best) {
+      best = cost;
+      P->res_cluster = C;
+      P->res_smem = smem;
+    }
+  }
+}
+
+bool fused_resident(const mcl_engine *e) {
+  const FusedPlan *P = e->fused;
+  return P && P->res_cluster && !P->asked && !P->skip_first_load && !e->zslab && e->d_dir[1] == nullptr;
+}
+
+bool fused_release_plan(mcl_engine *e) {
+  const bool asked = e->fused && e->fused->asked;
+  if (e->fused) e->fused->asked = false;
+  return asked;
+}
+
+int fused_resident_sweeps(mcl_engine *e, int n, bool measure) {
+  FusedPlan *P = e->fused;
+  ResidentArgs a;
+  a.reps = e->d_desc;
+  a.st = e->d_state;
+  a.dir = e->d_dir[e->cur];
+  a.sweep_ctr = e->d_sweep;
+  a.series = e->d_series;
+  a.series_len = e->d_series_len;
+  a.done = e->d_done;
+  a.n_sweeps = n;
+  a.measure = measure ? 1 : 0;
+  a.n_rep = e->n_rep;
+  a.adapt = (e->adapt && !e->d_mlp) ? 1 : 0;
+  CKF(resident_dispatch(e, a, resident_desc(e, P->res_cluster, P->res_smem)));
+  e->launches += 1;
+  return MCL_OK;
 }
 
 static FusedLaunch launch_desc(const mcl_engine *e, const FusedPlan *P) {

@@ -42,6 +42,7 @@
 #pragma once
 #include <type_traits>
 
+#include "sweep_draws.cuh"
 #include "sweep_fused.cuh"
 
 namespace mcl {
@@ -80,20 +81,6 @@ static __device__ __noinline__ void pass_ghosts(float *row0, long long cs, int p
   }
 }
 
-// Raw moments of two pairs of sites (lanes paired): m[0..5] = sum v_a v_b (xx, xy, xz, yy, yz, zz), m[6..8] = sum v.
-// Q and sum n follow per thread at the end: sum q_ab = 1.5 sum v_a v_b - 0.5 delta_ab (sites).
-__device__ __forceinline__ void pair_moments(float2 (&m)[9], const float2 (&u)[3], const float2 (&v)[3]) {
-  m[0] = __ffma2_rn(v[0], v[0], __fmul2_rn(u[0], u[0]));
-  m[1] = __ffma2_rn(v[0], v[1], __fmul2_rn(u[0], u[1]));
-  m[2] = __ffma2_rn(v[0], v[2], __fmul2_rn(u[0], u[2]));
-  m[3] = __ffma2_rn(v[1], v[1], __fmul2_rn(u[1], u[1]));
-  m[4] = __ffma2_rn(v[1], v[2], __fmul2_rn(u[1], u[2]));
-  m[5] = __ffma2_rn(v[2], v[2], __fmul2_rn(u[2], u[2]));
-  m[6] = __fadd2_rn(u[0], v[0]);
-  m[7] = __fadd2_rn(u[1], v[1]);
-  m[8] = __fadd2_rn(u[2], v[2]);
-}
-
 // Warp w of the CTA covers rows of parity w & 1: rows pc + 2 (RPW (w >> 1) + lane / NP), pair lane % NP.
 template <int TY, int TX, int NT>
 struct TaskMap {
@@ -107,28 +94,6 @@ struct TaskMap {
   }
   __device__ __forceinline__ static int pair(int tid) { return tid & (NP - 1); }
 };
-
-// Lane values of a pair draw (one Philox block for sites x and x + 2, non-flip models), bit-identical to
-// lane_draw(pair_half(out, 0), pair_half(out, 1), false).
-__device__ __forceinline__ float unit21_bits(uint32_t bits_shifted, uint32_t exponent) {
-  return __uint_as_float(exponent | (bits_shifted & 0x7FFFFCu));
-}
-__device__ __forceinline__ LaneDraw<float2> pair_draw_lanes(const U4 &o) {
-  LaneDraw<float2> r;
-  // u1 (angle field, bits 0..20 of lo): 2 u1 - 1 is used; keep u1 itself exact as (1 + f 2^-21) - 1
-  r.u1 = __fadd2_rn(make_float2(unit21_bits(o.x << 2, 0x3F800000u), unit21_bits(o.z << 2, 0x3F800000u)),
-                    make_float2(-1.f, -1.f));
-  // u3 (acceptance field, bits 10..30 of hi)
-  r.u3 = __fadd2_rn(make_float2(unit21_bits(o.y >> 8, 0x3F800000u), unit21_bits(o.w >> 8, 0x3F800000u)),
-                    make_float2(-1.f, -1.f));
-  r.u4 = make_float2(0.f, 0.f);
-  // axis field: bits 21..41 of the 64-bit half (lo, hi)
-  const uint32_t f0 = __funnelshift_r(o.x, o.y, 21) & 0x1FFFFFu, f1 = __funnelshift_r(o.z, o.w, 21) & 0x1FFFFFu;
-  r.w0 = make_float2(f0 < 698352u ? 1.f : 0.f, f1 < 698352u ? 1.f : 0.f);
-  r.w2 = make_float2(f0 >= 1396704u ? 1.f : 0.f, f1 >= 1396704u ? 1.f : 0.f);
-  r.w1 = make_float2(1.f - r.w0.x - r.w2.x, 1.f - r.w0.y - r.w2.y);
-  return r;
-}
 
 // An 8-byte shared-memory load the compiler may not merge with an earlier load of the same address (a merge would
 // keep the value in registers across the code between them).
@@ -340,14 +305,7 @@ __global__ void __launch_bounds__(NT, MINB) k_sweep_pass(ModelDev m, FusedArgs a
           pu[q] = *reinterpret_cast<const float2 *>(zu + q * PF);
           sx[q] = H == 0 ? oc[q * PF - 1] : oc[q * PF + 2];
         }
-        LaneDraw<float2> ld;
-        if (FLIP) {
-          const U4 u0 = site_draws(seed, sweep, ctr + H, 0), u1 = site_draws(seed, sweep, ctr + H + 2, 0);
-          ld = lane_draw(Draw{u0.x >> 8, u0.y >> 8, u0.z >> 8, u0.w >> 8},
-                         Draw{u1.x >> 8, u1.y >> 8, u1.z >> 8, u1.w >> 8}, true);
-        } else {
-          ld = pair_draw_lanes(site_draws(seed, sweep, ctr + H, 0));
-        }
+        const LaneDraw<float2> ld = pair_draws<FLIP>(seed, sweep, ctr + H);
         const V3<float2> n{o[0], o[1], o[2]};
         // +x / -x neighbour lanes: h = 0: +x = (jb, jb + 1), -x = (jb - 1, jb); h = 1: +x = (jb + 1, jb + 2),
         // -x = (jb, jb + 1)
@@ -374,7 +332,7 @@ __global__ void __launch_bounds__(NT, MINB) k_sweep_pass(ModelDev m, FusedArgs a
         w[4] = make_float2(wzu, wzu);
         w[5] = make_float2(wzd, wzd);
         const SiteResultT<float2> res =
-            site_update<POT, FLIP, PXY, CHIRAL, FIELD, float2, SINGLE>(m, n, nb, w, sid, sn, elecE, ld, av, T, invT);
+            site_update<POT, FLIP, PXY, CHIRAL, FIELD, float2, SINGLE, MEAS>(m, n, nb, w, sid, sn, elecE, ld, av, T, invT);
         // the other-parity pair again (not kept live across the physics): the colour-0 sites measured below and
         // the next plane's -z neighbours
 #pragma unroll
