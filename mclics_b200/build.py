@@ -21,10 +21,7 @@ EXE = os.path.join(HERE, "mclics_b200")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-O3", "--expt-relaxed-constexpr",
           "-I" + os.path.join(HERE, "..", "include")] + ARCH
-# the pair sweeps too: their paired FP32 operations round as written, whatever the compiler finds to contract around them
-PER_FILE = {"kernels_ref8.cu": ["-fmad=false"],
-            **{"sweep_%s_%s.cu" % (kind, pot): ["-fmad=false"] for kind in ("pass", "resident")
-               for pot in ("ll", "ghrl", "ghrl_chiral", "pear")}}
+PER_FILE = {"kernels_ref8.cu": ["-fmad=false"]}
 SOURCES = ["sweep_pass_ghrl.cu", "sweep_pass_ghrl_chiral.cu", "sweep_pass_pear.cu", "sweep_pass_ll.cu",
            "sweep_resident_ghrl.cu", "sweep_resident_ghrl_chiral.cu", "sweep_resident_pear.cu", "sweep_resident_ll.cu",
            "sweep_fused_ghrl.cu", "sweep_fused_pear.cu", "sweep_fused_ll.cu", "learned.cu", "kernels.cu",

@@ -41,6 +41,12 @@ __device__ __forceinline__ float neg_(float a) { return -a; }
 __device__ __forceinline__ float2 neg_(float2 a) { return make_float2(-a.x, -a.y); }
 __device__ __forceinline__ float sub_(float a, float b) { return __fadd_rn(a, -b); }
 __device__ __forceinline__ float2 sub_(float2 a, float2 b) { return __fadd2_rn(a, neg_(b)); }
+// a - b that is not contracted with a multiplication feeding it: ptxas fuses a paired product into a paired sum
+// whatever the front end's -fmad says, but not into two single ones.
+__device__ __forceinline__ float sub_apart(float a, float b) { return sub_(a, b); }
+__device__ __forceinline__ float2 sub_apart(float2 a, float2 b) {
+  return make_float2(__fadd_rn(a.x, -b.x), __fadd_rn(a.y, -b.y));
+}
 template <typename L>
 __device__ __forceinline__ L splat(float v);
 template <>
@@ -134,35 +140,37 @@ __device__ __forceinline__ L bond(const ModelDev &m, const V3<L> &x, const V3<L>
 }
 
 // Bond sums of one or two directors over the six bonds, with weights w[d] in {0, 1} (0: free edge or empty
-// site). PXY = true: the x and y neighbours are known to be present, their weights are not applied (exact: the
-// weight would be 1). The two-director form evaluates both in one pass, so each neighbour is used once.
-template <int POT, bool PXY, bool CHIRAL, int D, typename L>
+// site). PRES names the neighbours known to be present, whose weights are not applied (exact: the weight would be 1):
+// kPresentXY those along x and y, kPresentZ those along z. The two-director form evaluates both in one pass, so each neighbour is used once.
+constexpr int kPresentXY = 1, kPresentZ = 2;
+__host__ __device__ constexpr bool present(int pres, int d) { return (pres & (d < 4 ? kPresentXY : kPresentZ)) != 0; }
+template <int POT, int PRES, bool CHIRAL, int D, typename L>
 __device__ __forceinline__ L acc_bond(const ModelDev &m, const V3<L> &x, const V3<L> &y, const L &w, const L &e) {
   const L u = bond<POT, D, CHIRAL>(m, x, y);
-  if (PXY && D < 4) return D == 0 ? u : add_(e, u);
+  if (present(PRES, D)) return D == 0 ? u : add_(e, u);
   return D == 0 ? mul_(w, u) : fma_(w, u, e);
 }
 
 // Lebwohl-Lasher sums: sum_j w_j (n.n_j)^2 over the six bonds, then one multiplication by -1.5 A (the bond
 // energy is that constant times a square, so it factors out of the sum).
-template <bool PXY, int D, typename L>
+template <int PRES, int D, typename L>
 __device__ __forceinline__ L ll_acc(const V3<L> &x, const V3<L> &y, const L &w, const L &s) {
   const L b = dot(x, y);
-  if (PXY && D < 4) return D == 0 ? mul_(b, b) : fma_(b, b, s);
+  if (present(PRES, D)) return D == 0 ? mul_(b, b) : fma_(b, b, s);
   return D == 0 ? mul_(mul_(w, b), b) : fma_(mul_(w, b), b, s);
 }
-template <bool PXY, typename L>
+template <int PRES, typename L>
 __device__ __forceinline__ L ll_sum_raw(const V3<L> &x, const V3<L> (&nb)[6], const L (&w)[6]) {
-  L s = ll_acc<PXY, 0>(x, nb[0], w[0], w[0]);
-  s = ll_acc<PXY, 1>(x, nb[1], w[1], s);
-  s = ll_acc<PXY, 2>(x, nb[2], w[2], s);
-  s = ll_acc<PXY, 3>(x, nb[3], w[3], s);
-  s = ll_acc<PXY, 4>(x, nb[4], w[4], s);
-  return ll_acc<PXY, 5>(x, nb[5], w[5], s);
+  L s = ll_acc<PRES, 0>(x, nb[0], w[0], w[0]);
+  s = ll_acc<PRES, 1>(x, nb[1], w[1], s);
+  s = ll_acc<PRES, 2>(x, nb[2], w[2], s);
+  s = ll_acc<PRES, 3>(x, nb[3], w[3], s);
+  s = ll_acc<PRES, 4>(x, nb[4], w[4], s);
+  return ll_acc<PRES, 5>(x, nb[5], w[5], s);
 }
-template <bool PXY, typename L>
+template <int PRES, typename L>
 __device__ __forceinline__ L ll_sum(const ModelDev &m, const V3<L> &x, const V3<L> (&nb)[6], const L (&w)[6]) {
-  return mul_(splat<L>(-1.5f * m.A), ll_sum_raw<PXY>(x, nb, w));
+  return mul_(splat<L>(-1.5f * m.A), ll_sum_raw<PRES>(x, nb, w));
 }
 
 // GHRL without the chiral term as sums over the site's bonds. With a_i = n.r, a_j = n_j.r, b = n.n_j, the pair
@@ -173,7 +181,7 @@ __device__ __forceinline__ L ll_sum(const ModelDev &m, const V3<L> &x, const V3<
 // (A_a = 1.5 a_i,a^2, B = b^2; an absent bond has w = 0, applied by scaling b and A + K). NS directors (1: one
 // site energy; 2: the old and new director of a trial) go through the bonds together, so each neighbour and its
 // K_d are used by both and then released.
-template <bool PXY, int NS, typename L>
+template <int PRES, int NS, typename L>
 __device__ __forceinline__ void ghrl_sums(const ModelDev &m, const V3<L> *const (&x)[NS], const V3<L> (&nb)[6],
                                           const L (&w)[6], L (&out)[NS]) {
   const L h3 = splat<L>(1.5f), r15 = splat<L>(1.5f * m.rho), lamp = splat<L>(fmaf(-0.5f, m.rho, m.lam));
@@ -194,7 +202,7 @@ __device__ __forceinline__ void ghrl_sums(const ModelDev &m, const V3<L> *const 
 #pragma unroll
       for (int i = 0; i < NS; i++) {
         L b = dot(*x[i], nb[d]), t = add_(A[i], K);
-        if (!(PXY && d < 4)) {
+        if (!present(PRES, d)) {
           b = mul_(w[d], b);
           t = mul_(w[d], t);
         }
@@ -210,46 +218,46 @@ __device__ __forceinline__ void ghrl_sums(const ModelDev &m, const V3<L> *const 
       e[i] = fma_(mul_(splat<L>(m.mu), ai), mab[i], e[i]);
     }
   }
-  const L nw = PXY ? add_(add_(w[4], w[5]), splat<L>(4.f))
-                   : add_(add_(add_(w[0], w[1]), add_(w[2], w[3])), add_(w[4], w[5]));
+  const L nxy = (PRES & kPresentXY) ? splat<L>(4.f) : add_(add_(w[0], w[1]), add_(w[2], w[3]));  // exact in any order
+  const L nw = (PRES & kPresentZ) ? add_(nxy, splat<L>(2.f)) : add_(nxy, add_(w[4], w[5]));
   const L c = mul_(splat<L>(m.ghrl_c0), nw);
 #pragma unroll
   for (int i = 0; i < NS; i++) out[i] = fma_(splat<L>(1.5f * m.nu), sB[i], add_(e[i], c));
 }
 
-template <int POT, bool PXY, bool CHIRAL, typename L>
+template <int POT, int PRES, bool CHIRAL, typename L>
 __device__ __forceinline__ L bond_sum(const ModelDev &m, const V3<L> &x, const V3<L> (&nb)[6], const L (&w)[6]) {
-  if (POT == POT_LL) return ll_sum<PXY>(m, x, nb, w);
+  if (POT == POT_LL) return ll_sum<PRES>(m, x, nb, w);
   if (POT == POT_GHRL && !CHIRAL) {
     const V3<L> *const xs[1] = {&x};
     L out[1];
-    ghrl_sums<PXY, 1>(m, xs, nb, w, out);
+    ghrl_sums<PRES, 1>(m, xs, nb, w, out);
     return out[0];
   }
-  L e = acc_bond<POT, PXY, CHIRAL, 0>(m, x, nb[0], w[0], w[0]);
-  e = acc_bond<POT, PXY, CHIRAL, 1>(m, x, nb[1], w[1], e);
-  e = acc_bond<POT, PXY, CHIRAL, 2>(m, x, nb[2], w[2], e);
-  e = acc_bond<POT, PXY, CHIRAL, 3>(m, x, nb[3], w[3], e);
-  e = acc_bond<POT, PXY, CHIRAL, 4>(m, x, nb[4], w[4], e);
-  e = acc_bond<POT, PXY, CHIRAL, 5>(m, x, nb[5], w[5], e);
+  L e = acc_bond<POT, PRES, CHIRAL, 0>(m, x, nb[0], w[0], w[0]);
+  e = acc_bond<POT, PRES, CHIRAL, 1>(m, x, nb[1], w[1], e);
+  e = acc_bond<POT, PRES, CHIRAL, 2>(m, x, nb[2], w[2], e);
+  e = acc_bond<POT, PRES, CHIRAL, 3>(m, x, nb[3], w[3], e);
+  e = acc_bond<POT, PRES, CHIRAL, 4>(m, x, nb[4], w[4], e);
+  e = acc_bond<POT, PRES, CHIRAL, 5>(m, x, nb[5], w[5], e);
   return e;
 }
 
-template <int POT, bool PXY, bool CHIRAL, typename L>
+template <int POT, int PRES, bool CHIRAL, typename L>
 __device__ __forceinline__ void bond_sum2(const ModelDev &m, const V3<L> &x, const V3<L> &x2, const V3<L> (&nb)[6],
                                           const L (&w)[6], L &e1, L &e2) {
   if (POT == POT_LL) {
-    L s1 = ll_acc<PXY, 0>(x, nb[0], w[0], w[0]), s2 = ll_acc<PXY, 0>(x2, nb[0], w[0], w[0]);
-    s1 = ll_acc<PXY, 1>(x, nb[1], w[1], s1);
-    s2 = ll_acc<PXY, 1>(x2, nb[1], w[1], s2);
-    s1 = ll_acc<PXY, 2>(x, nb[2], w[2], s1);
-    s2 = ll_acc<PXY, 2>(x2, nb[2], w[2], s2);
-    s1 = ll_acc<PXY, 3>(x, nb[3], w[3], s1);
-    s2 = ll_acc<PXY, 3>(x2, nb[3], w[3], s2);
-    s1 = ll_acc<PXY, 4>(x, nb[4], w[4], s1);
-    s2 = ll_acc<PXY, 4>(x2, nb[4], w[4], s2);
-    s1 = ll_acc<PXY, 5>(x, nb[5], w[5], s1);
-    s2 = ll_acc<PXY, 5>(x2, nb[5], w[5], s2);
+    L s1 = ll_acc<PRES, 0>(x, nb[0], w[0], w[0]), s2 = ll_acc<PRES, 0>(x2, nb[0], w[0], w[0]);
+    s1 = ll_acc<PRES, 1>(x, nb[1], w[1], s1);
+    s2 = ll_acc<PRES, 1>(x2, nb[1], w[1], s2);
+    s1 = ll_acc<PRES, 2>(x, nb[2], w[2], s1);
+    s2 = ll_acc<PRES, 2>(x2, nb[2], w[2], s2);
+    s1 = ll_acc<PRES, 3>(x, nb[3], w[3], s1);
+    s2 = ll_acc<PRES, 3>(x2, nb[3], w[3], s2);
+    s1 = ll_acc<PRES, 4>(x, nb[4], w[4], s1);
+    s2 = ll_acc<PRES, 4>(x2, nb[4], w[4], s2);
+    s1 = ll_acc<PRES, 5>(x, nb[5], w[5], s1);
+    s2 = ll_acc<PRES, 5>(x2, nb[5], w[5], s2);
     e1 = mul_(splat<L>(-1.5f * m.A), s1);
     e2 = mul_(splat<L>(-1.5f * m.A), s2);
     return;
@@ -257,23 +265,23 @@ __device__ __forceinline__ void bond_sum2(const ModelDev &m, const V3<L> &x, con
   if (POT == POT_GHRL && !CHIRAL) {
     const V3<L> *const xs[2] = {&x, &x2};
     L out[2];
-    ghrl_sums<PXY, 2>(m, xs, nb, w, out);
+    ghrl_sums<PRES, 2>(m, xs, nb, w, out);
     e1 = out[0];
     e2 = out[1];
     return;
   }
-  e1 = acc_bond<POT, PXY, CHIRAL, 0>(m, x, nb[0], w[0], w[0]);
-  e2 = acc_bond<POT, PXY, CHIRAL, 0>(m, x2, nb[0], w[0], w[0]);
-  e1 = acc_bond<POT, PXY, CHIRAL, 1>(m, x, nb[1], w[1], e1);
-  e2 = acc_bond<POT, PXY, CHIRAL, 1>(m, x2, nb[1], w[1], e2);
-  e1 = acc_bond<POT, PXY, CHIRAL, 2>(m, x, nb[2], w[2], e1);
-  e2 = acc_bond<POT, PXY, CHIRAL, 2>(m, x2, nb[2], w[2], e2);
-  e1 = acc_bond<POT, PXY, CHIRAL, 3>(m, x, nb[3], w[3], e1);
-  e2 = acc_bond<POT, PXY, CHIRAL, 3>(m, x2, nb[3], w[3], e2);
-  e1 = acc_bond<POT, PXY, CHIRAL, 4>(m, x, nb[4], w[4], e1);
-  e2 = acc_bond<POT, PXY, CHIRAL, 4>(m, x2, nb[4], w[4], e2);
-  e1 = acc_bond<POT, PXY, CHIRAL, 5>(m, x, nb[5], w[5], e1);
-  e2 = acc_bond<POT, PXY, CHIRAL, 5>(m, x2, nb[5], w[5], e2);
+  e1 = acc_bond<POT, PRES, CHIRAL, 0>(m, x, nb[0], w[0], w[0]);
+  e2 = acc_bond<POT, PRES, CHIRAL, 0>(m, x2, nb[0], w[0], w[0]);
+  e1 = acc_bond<POT, PRES, CHIRAL, 1>(m, x, nb[1], w[1], e1);
+  e2 = acc_bond<POT, PRES, CHIRAL, 1>(m, x2, nb[1], w[1], e2);
+  e1 = acc_bond<POT, PRES, CHIRAL, 2>(m, x, nb[2], w[2], e1);
+  e2 = acc_bond<POT, PRES, CHIRAL, 2>(m, x2, nb[2], w[2], e2);
+  e1 = acc_bond<POT, PRES, CHIRAL, 3>(m, x, nb[3], w[3], e1);
+  e2 = acc_bond<POT, PRES, CHIRAL, 3>(m, x2, nb[3], w[3], e2);
+  e1 = acc_bond<POT, PRES, CHIRAL, 4>(m, x, nb[4], w[4], e1);
+  e2 = acc_bond<POT, PRES, CHIRAL, 4>(m, x2, nb[4], w[4], e2);
+  e1 = acc_bond<POT, PRES, CHIRAL, 5>(m, x, nb[5], w[5], e1);
+  e2 = acc_bond<POT, PRES, CHIRAL, 5>(m, x2, nb[5], w[5], e2);
 }
 
 // Field, src/potential.cpp:59-63.
@@ -367,8 +375,14 @@ __device__ __forceinline__ void sincos_pi(float2 va, float2 &s, float2 &c) {
   sincos_pi(va.x, s.x, c.x);
   sincos_pi(va.y, s.y, c.y);
 }
-__device__ __forceinline__ float rsqrt_(float a) { return rsqrtf(a); }
-__device__ __forceinline__ float2 rsqrt_(float2 a) { return make_float2(rsqrtf(a.x), rsqrtf(a.y)); }
+// Reciprocal square root of a squared length near 1: the hardware instruction, without the scaling of denormal
+// arguments around it (the same bits for every normal argument).
+__device__ __forceinline__ float rsqrt_(float a) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ float2 rsqrt_(float2 a) { return make_float2(rsqrt_(a.x), rsqrt_(a.y)); }
 
 // Trial rotation by pi * va about axis `axis` (src/evolve.cpp:153-176): the reference's three rotations in one
 // branch-free Rodrigues form n' = c n + (1 - c) n_a e_a - s (e_a x n), then renormalised. w0..w2: one-hot axis.
@@ -433,28 +447,28 @@ __device__ __forceinline__ V3<L> sel3(LB<L> c, const V3<L> &a, const V3<L> &b) {
 }
 
 // One trial move (src/evolve.cpp:133-207): rotation, Metropolis, then the optional n -> -n trial.
-// Compile-time features: FLIP (n -> -n trial), PXY (x, y neighbours always present), CHIRAL (GHRL sigma term),
+// Compile-time features: FLIP (n -> -n trial), PRES (neighbours always present), CHIRAL (GHRL sigma term),
 // FIELD (field term), SINGLE = false (the caller knows the site has no single-site term: no surface, no field;
 // the energies are then the bond sums themselves, which is what adding the zero single term gives, up to the sign
 // of a zero). Every combination rounds like the general one on the inputs it applies to.
-template <int POT, bool FLIP, bool PXY, bool CHIRAL, bool FIELD, typename L, bool SINGLE = true, bool ENERGY = true>
+template <int POT, bool FLIP, int PRES, bool CHIRAL, bool FIELD, typename L, bool SINGLE = true, bool FUSED = false>
 __device__ __forceinline__ SiteResultT<L> site_update(const ModelDev &m, const V3<L> &n, const V3<L> (&nb)[6],
                                                       const L (&w)[6], int sid, const Vec3 &s, float elecE,
                                                       const LaneDraw<L> &d, float av, float T, float invT) {
   const L va = mul_(fma_(splat<L>(2.f), d.u1, splat<L>(-1.f)), splat<L>(av));
   const V3<L> nn = rotate_trial(n, va, d.w0, d.w1, d.w2);
   L b_old, b_new;
-  bond_sum2<POT, PXY, CHIRAL>(m, n, nn, nb, w, b_old, b_new);
+  bond_sum2<POT, PRES, CHIRAL>(m, n, nn, nb, w, b_old, b_new);
   const L s_old = SINGLE ? single_energy<FIELD>(m, n, sid, s, elecE) : splat<L>(0.f);
   const L s_new = SINGLE ? single_energy<FIELD>(m, nn, sid, s, elecE) : splat<L>(0.f);
   const L e_old = SINGLE ? add_(b_old, s_old) : b_old, e_new = SINGLE ? add_(b_new, s_new) : b_new;
   SiteResultT<L> r;
   L dE;
-  if (POT == POT_LL && !SINGLE && !ENERGY) {
+  if (POT == POT_LL && FUSED) {
     const L c = splat<L>(-1.5f * m.A);
-    dE = fma_(c, ll_sum_raw<PXY>(nn, nb, w), neg_(mul_(c, ll_sum_raw<PXY>(n, nb, w))));
+    dE = fma_(c, ll_sum_raw<PRES>(nn, nb, w), neg_(mul_(c, ll_sum_raw<PRES>(n, nb, w))));
   } else {
-    dE = sub_(e_new, e_old);
+    dE = POT == POT_LL ? sub_apart(e_new, e_old) : sub_(e_new, e_old);
   }
   r.rot = metropolis(d.u3, dE, invT, T);
   r.n = sel3<L>(r.rot, nn, n);
@@ -462,7 +476,7 @@ __device__ __forceinline__ SiteResultT<L> site_update(const ModelDev &m, const V
   r.single = SINGLE ? sel_(r.rot, s_new, s_old) : splat<L>(0.f);
   if (FLIP) {
     const V3<L> f{neg_(r.n.x), neg_(r.n.y), neg_(r.n.z)};
-    const L bf = bond_sum<POT, PXY, CHIRAL>(m, f, nb, w);
+    const L bf = bond_sum<POT, PRES, CHIRAL>(m, f, nb, w);
     const L sf = SINGLE ? single_energy<FIELD>(m, f, sid, s, elecE) : splat<L>(0.f);
     const L e_cur = SINGLE ? add_(r.bond, r.single) : r.bond;
     r.flip = metropolis(d.u4, SINGLE ? sub_(add_(bf, sf), e_cur) : sub_(bf, e_cur), invT, T);

@@ -1,4 +1,5 @@
-// What the sweeps on pairs of sites share (colour passes, resident sweep): the draws of a pair and its raw moments.
+// What the sweeps on pairs of sites share (colour passes, resident sweep): the draws of a pair, its raw
+// moments and their sums over a warp.
 #pragma once
 #include "common.cuh"
 #include "physics.cuh"
@@ -50,6 +51,26 @@ __device__ __forceinline__ void pair_moments(float2 (&m)[9], const float2 (&u)[3
   m[6] = __fadd2_rn(u[0], v[0]);
   m[7] = __fadd2_rn(u[1], v[1]);
   m[8] = __fadd2_rn(u[2], v[2]);
+}
+
+// Sums of ten values over a warp: the halves of the warp split the values between them at every step (12 double
+// shuffles instead of 50). The lane that holds value k afterwards returns k, the others -1.
+__device__ __forceinline__ int warp_sum10(const double (&v)[kPartials], double &out) {
+  const int lane = threadIdx.x & 31;
+  const bool b16 = lane & 16, b8 = lane & 8, b4 = lane & 4, b2 = lane & 2;
+  double a[6], b[4], c[2];
+#pragma unroll
+  for (int i = 0; i < 5; i++) a[i] = (b16 ? v[5 + i] : v[i]) + __shfl_xor_sync(0xffffffffu, b16 ? v[i] : v[5 + i], 16);
+  a[5] = 0.0;
+#pragma unroll
+  for (int i = 0; i < 3; i++) b[i] = (b8 ? a[3 + i] : a[i]) + __shfl_xor_sync(0xffffffffu, b8 ? a[i] : a[3 + i], 8);
+  b[3] = 0.0;
+#pragma unroll
+  for (int i = 0; i < 2; i++) c[i] = (b4 ? b[2 + i] : b[i]) + __shfl_xor_sync(0xffffffffu, b4 ? b[i] : b[2 + i], 4);
+  double d = (b2 ? c[1] : c[0]) + __shfl_xor_sync(0xffffffffu, b2 ? c[0] : c[1], 2);
+  out = d + __shfl_xor_sync(0xffffffffu, d, 1);
+  const int in4 = (b4 ? 2 : 0) + (b2 ? 1 : 0), in8 = (b8 ? 3 : 0) + in4;
+  return (lane & 1) == 0 && in4 < 3 && in8 < 5 ? (b16 ? 5 : 0) + in8 : -1;
 }
 
 }  // namespace mcl

@@ -83,45 +83,101 @@ static int encode_map(CUtensorMap *map, float *base, const RepDesc &D, int cells
     if (e_ != cudaSuccess) return cuda_fail(e_, #call);  \
   } while (0)
 
-// Tile and segment choice for configuration `cfg`: z segments sized so that the number of work items is close to
-// a multiple of the resident CTAs, with segments long enough that the extra planes of each stay cheap (fused: four
-// loaded, two of them computed; colour pass: two loaded).
+// Colour passes: what a plane costs a CTA, in us, by model (Lebwohl-Lasher, GHRL, chiral GHRL, models with flips) and
+// configuration (2, 3, 4): `issue` times the CTAs that share an SM, but at least `chain`, the latency of one plane. From
+// sweeps of lattices between 64^3 and 256^3 over all configurations and 2-24 planes per segment.
+struct PassCost {
+  double issue[3], chain[3];
+};
+static const PassCost kPassCost[4] = {{{0.76, 0.85, 0.43}, {1.05, 1.05, 1.00}},
+                                      {{1.08, 1.02, 0.456}, {1.50, 1.46, 1.25}},
+                                      {{1.20, 1.25, 0.62}, {1.60, 1.30, 1.05}},
+                                      {{1.58, 1.40, 0.80}, {2.90, 2.08, 2.20}}};
+
+static int pass_model(const mcl_engine *e) {
+  if (e->model.flip != 0 || e->model.potential == POT_PEAR) return 3;
+  if (e->model.potential == POT_GHRL) return e->model.sigma != 0.f ? 2 : 1;
+  return 0;
+}
+
+static long long tiles_of(const mcl_engine *e, const FusedCfg &C) {
+  long long tiles = 0;
+  for (const auto &D : e->desc) tiles += (long long)((D.nx + C.tx - 1) / C.tx) * ((D.ny + C.ty - 1) / C.ty);
+  return tiles;
+}
+
+// Expected time of one colour pass in us: 3.8 us of launch and first planes, then the planes of a segment for every wave
+// of CTAs (the last wave counts half when it is not full: CTAs are handed out as they end).
+static double pass_time(const mcl_engine *e, int cfg, int seg, int sms) {
+  const FusedCfg &C = kCfgs[cfg];
+  const PassCost &K = kPassCost[pass_model(e)];
+  long long items = 0;
+  for (const auto &D : e->desc)
+    items += (long long)((D.nx + C.tx - 1) / C.tx) * ((D.ny + C.ty - 1) / C.ty) * ((D.nz + seg - 1) / seg);
+  const double slots = (double)C.ctas_per_sm * sms, waves = items / slots;
+  const double share = std::min<double>(C.ctas_per_sm, std::ceil((double)items / sms));
+  const double plane = std::max(K.chain[cfg - 2], K.issue[cfg - 2] * share);
+  return 3.8 + (waves <= 1 ? seg : (seg + 1.2) * std::max(waves, std::ceil(waves) - 0.5)) * plane;
+}
+
+// Segment choice for configuration `cfg`. Fused kernel and learned passes: segments sized so that the number of work
+// items is close to a multiple of the resident CTAs, and long enough that the extra planes of each stay cheap (fused:
+// four loaded, two of them computed; learned pass: two loaded). Colour passes: the shortest expected pass over 2-15
+// planes. Per sweep in us, unmeasured / measured, with the work-item rule for both and configuration 2 (3 with flips)
+// -> with the shortest pass over configurations too: LL 64^3 29.1 / 33.2 -> 16.8 / 18.9, LL 100^3 37.0 / 41.4 ->
+// 31.9 / 35.5, GHRL slab 128^3 54.9 / 63.5 -> 46.5 / 52.8, 256^3 240 / 274 -> 215 / 240, chiral 101 x 75 x 50
+// 35.2 / 39.4 -> 22.9 / 26.0, pear slab 64^3 41.3 / 45.5 -> 20.9 / 25.1.
 static void choose_segments(const mcl_engine *e, FusedPlan &P, int sms) {
   const FusedCfg &C = P.C;
   P.tx = C.tx;
   P.ty = C.ty;
-  long long tiles = 0, maxz = 1;
-  for (auto &D : e->desc) {
-    tiles += (long long)((D.nx + P.tx - 1) / P.tx) * ((D.ny + P.ty - 1) / P.ty);
-    maxz = std::max<long long>(maxz, D.nz);
-  }
-  const long long slots = (long long)C.ctas_per_sm * sms;
-  int best = 1;
-  double best_score = -1;
-  for (int nseg = 1; nseg <= 256; nseg++) {
-    const double seg_len = (double)maxz / nseg;
-    if (seg_len < 6 && nseg > 1) break;
-    const long long items = tiles * nseg;
-    const double waves = (double)items / slots;
-    const double eff = waves / std::ceil(waves);
-    const double extra = C.kind ? 2.0 * 0.15 : 4.0 * 0.35;  // extra planes mostly hit L2
-    const double score = eff * seg_len / (seg_len + extra);
-    if (score > best_score + 1e-9) {
-      best_score = score;
-      best = nseg;
+  long long maxz = 1;
+  for (auto &D : e->desc) maxz = std::max<long long>(maxz, D.nz);
+  if (C.kind == 1 && !P.learned) {
+    P.seg = (int)std::min<long long>(2, maxz);
+    for (int seg = 3; seg <= 15 && seg <= maxz; seg++)
+      if (pass_time(e, P.cfg, seg, sms) < pass_time(e, P.cfg, P.seg, sms)) P.seg = seg;
+  } else {
+    const long long tiles = tiles_of(e, C), slots = (long long)C.ctas_per_sm * sms;
+    int best = 1;
+    double best_score = -1;
+    for (int nseg = 1; nseg <= 256; nseg++) {
+      const double seg_len = (double)maxz / nseg;
+      if (seg_len < 6 && nseg > 1) break;
+      const double waves = (double)(tiles * nseg) / slots;
+      const double eff = waves / std::ceil(waves);
+      const double extra = C.kind ? 2.0 * 0.15 : 4.0 * 0.35;  // extra planes mostly hit L2
+      const double score = eff * seg_len / (seg_len + extra);
+      if (score > best_score + 1e-9) {
+        best_score = score;
+        best = nseg;
+      }
     }
+    P.seg = (int)((maxz + best - 1) / best);
   }
-  P.seg = (int)((maxz + best - 1) / best);
   if (P.seg_override > 0) P.seg = (int)std::min<long long>(P.seg_override, maxz);
 }
 
+// The colour passes (faster than the fused kernel on every measured workload) in the configuration with the shortest
+// expected pass.
 static int choose_cfg(const mcl_engine *e) {
-  // Colour passes (faster than the fused kernel on every measured workload): 3 CTAs per SM fit the 80 registers
-  // of the non-flip kernels; flip models (a second trial per site) need the 2-CTA variant's registers.
   const char *env = getenv("MCL_FUSED_CFG");
   if (env) return std::max(0, std::min(kNumCfgs - 1, atoi(env)));
-  const bool flip = e->model.flip != 0 || e->model.potential == POT_PEAR;
-  return flip ? 3 : 2;
+  int sms = 148, best = 2;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
+  double best_time = 1e30;
+  for (int cfg = 2; cfg < kNumCfgs; cfg++) {
+    FusedPlan P;
+    P.cfg = cfg;
+    P.C = kCfgs[cfg];
+    choose_segments(e, P, sms);
+    const double t = pass_time(e, cfg, P.seg, sms);
+    if (t < best_time) {
+      best_time = t;
+      best = cfg;
+    }
+  }
+  return best;
 }
 
 static int prepare_kernel(mcl_engine *e, FusedPlan *P);
@@ -262,15 +318,14 @@ void fused_plan_candidates(const mcl_engine *e, std::vector<std::pair<int, int>>
     std::vector<int> segs = {P.seg, P.seg * 2, (P.seg + 1) / 2, maxz};
     // lattices too small to give every SM a work item (C1's 32^3: 10 items) also try short segments in the colour
     // passes, which trade two extra planes per item for more items in flight
-    long long tiles = 0;
-    for (auto &D : e->desc) tiles += (long long)((D.nx + P.tx - 1) / P.tx) * ((D.ny + P.ty - 1) / P.ty);
+    const long long tiles = tiles_of(e, P.C);
     const bool few = P.C.kind == 1 && tiles * ((maxz + P.seg - 1) / P.seg) < sms;
     if (few)
       for (int sg : {2, 3, 4}) segs.push_back(sg);
     std::sort(segs.begin(), segs.end());
     segs.erase(std::unique(segs.begin(), segs.end()), segs.end());
     for (int sg : segs)
-      if (sg >= 6 || sg == maxz || (few && sg >= 2)) out.push_back({cfg, std::min(sg, maxz)});
+      if (sg >= 6 || sg == P.seg || sg == maxz || (few && sg >= 2)) out.push_back({cfg, std::min(sg, maxz)});
   }
   std::sort(out.begin(), out.end());
   out.erase(std::unique(out.begin(), out.end()), out.end());
@@ -390,27 +445,22 @@ static int clusters_that_fit(const mcl_engine *e, int C) {
 //   LL 64 x 24^3      15.1 / 18.4         25.4 / 30.2    44.2 / 74.9    37.5 / 41.0
 //   LL 128 x 16^3     14.4 / 20.0         28.0 / 40.5    62.6 / 86.9    30.8 / 33.0
 // A colour costs a chain of one task or the issue of the tasks of a full CTA, `round` us per 512, and a cluster barrier
-// that grows with C; replicas beyond the clusters that fit the device (33, 15 and 7) wait for a free one. The colour
-// passes cost three launches (14.4 us) or the same rounds over all SMs.
+// that grows with C; replicas beyond the clusters that fit the device (33, 15 and 7) wait for a free one.
 static void resident_choose(const mcl_engine *e, FusedPlan *P) {
   P->res_cluster = 0;
-  const bool flip = e->model.flip != 0 || e->model.potential == POT_PEAR;
-  const bool chiral = e->model.potential == POT_GHRL && e->model.sigma != 0.f;
-  const double round = (flip ? (e->model.potential == POT_LL ? 2.2 : 3.3) : chiral ? 2.4 : e->model.potential == POT_GHRL ? 1.9 : 1.45);
+  static const double kRound[4] = {1.45, 1.9, 2.4, 3.3};  // by pass_model
+  const double round = kRound[pass_model(e)];
   int min_nz = 1 << 30, sms = 148;
-  double all_tasks = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
-  for (const auto &D : e->desc) {
-    min_nz = std::min(min_nz, D.nz);
-    all_tasks += (double)D.nz * D.ny * res_pairs(D.nx);
-  }
+  for (const auto &D : e->desc) min_nz = std::min(min_nz, D.nz);
   ResidentLaunch limits = resident_desc(e, 1, 0);
   limits.prepare = true;
   if (resident_dispatch(e, ResidentArgs{}, limits) != cudaSuccess) {
     cudaGetLastError();  // this combination of options has no kernel
     return;
   }
-  double best = std::max(flip ? 22.0 : 14.4, 6.0 + 2.0 * round * 1.1 * all_tasks / ((double)kResThreads * sms));
+  if (P->C.kind != 1) return;
+  double best = 5.0 + 2.0 * pass_time(e, P->cfg, P->seg, sms);  // the finalisation and the gaps between three launches
   for (int C = 1; C <= kResMaxC && C <= min_nz; C *= 2) {
     size_t smem = 0;
     for (const auto &D : e->desc)

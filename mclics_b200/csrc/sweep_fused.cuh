@@ -213,7 +213,8 @@ __device__ __forceinline__ void pair_task(const ModelDev &m, const Ctx &c, float
   w[4] = make_float2(wzu, wzu);
   w[5] = make_float2(wzd, wzd);
   const SiteResultT<float2> r =
-      site_update<POT, FLIP, PXY, CHIRAL, FIELD, float2>(m, n, nb, w, sid, sn, c.elecE, ld, c.av, c.T, c.invT);
+      site_update<POT, FLIP, PXY ? kPresentXY : 0, CHIRAL, FIELD, float2>(m, n, nb, w, sid, sn, c.elecE, ld, c.av, c.T,
+                                                                          c.invT);
   const float2 nx2[3] = {r.n.x, r.n.y, r.n.z};
   // Only the updated lanes go back: along a periodic x with nx % 4 == 2 the right ring site shares its pair of cells
   // with the tile's last row pair, whose second lane is outside the lattice — two tasks, one lane each.

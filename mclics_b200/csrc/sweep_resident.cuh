@@ -98,26 +98,6 @@ __device__ __forceinline__ void st_cluster(unsigned addr, double v) {
   asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
 }
 
-// Sums of ten values over a warp: the halves of the warp split the values between them at every step (12 double
-// shuffles instead of 50). The lane that holds value k afterwards returns k, the others -1.
-__device__ __forceinline__ int warp_sum10(const double (&v)[kPartials], double &out) {
-  const int lane = threadIdx.x & 31;
-  const bool b16 = lane & 16, b8 = lane & 8, b4 = lane & 4, b2 = lane & 2;
-  double a[6], b[4], c[2];
-#pragma unroll
-  for (int i = 0; i < 5; i++) a[i] = (b16 ? v[5 + i] : v[i]) + __shfl_xor_sync(0xffffffffu, b16 ? v[i] : v[5 + i], 16);
-  a[5] = 0.0;
-#pragma unroll
-  for (int i = 0; i < 3; i++) b[i] = (b8 ? a[3 + i] : a[i]) + __shfl_xor_sync(0xffffffffu, b8 ? a[i] : a[3 + i], 8);
-  b[3] = 0.0;
-#pragma unroll
-  for (int i = 0; i < 2; i++) c[i] = (b4 ? b[2 + i] : b[i]) + __shfl_xor_sync(0xffffffffu, b4 ? b[i] : b[2 + i], 4);
-  double d = (b2 ? c[1] : c[0]) + __shfl_xor_sync(0xffffffffu, b2 ? c[0] : c[1], 2);
-  out = d + __shfl_xor_sync(0xffffffffu, d, 1);
-  const int in4 = (b4 ? 2 : 0) + (b2 ? 1 : 0), in8 = (b8 ? 3 : 0) + in4;
-  return (lane & 1) == 0 && in4 < 3 && in8 < 5 ? (b16 ? 5 : 0) + in8 : -1;
-}
-
 template <int POT, bool SLAB, bool FLIP, bool PXY, bool CHIRAL, bool FIELD>
 __global__ void __launch_bounds__(kResThreads, 1) k_sweep_resident(ModelDev m, ResidentArgs a) {
   extern __shared__ __align__(16) unsigned char res_smem[];
@@ -260,12 +240,13 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweep_resident(ModelDev m, R
           const float wu = (perz || z + 1 < nz) ? 1.f : 0.f, wd = (perz || z > 0) ? 1.f : 0.f;
           w[4] = make_float2(wu, wu);
           w[5] = make_float2(wd, wd);
+          constexpr int PRES = PXY ? kPresentXY : 0;
           if (SLAB || FIELD || POT != POT_LL || meas)
-            res = site_update<POT, FLIP, PXY, CHIRAL, FIELD, float2, SLAB || FIELD>(m, n, nb, w, sid, sn, elecE, ld, av,
-                                                                                     T, invT);
+            res = site_update<POT, FLIP, PRES, CHIRAL, FIELD, float2, SLAB || FIELD>(m, n, nb, w, sid, sn, elecE, ld, av,
+                                                                                      T, invT);
           else  // the difference as the unmeasured colour pass rounds it
-            res = site_update<POT, FLIP, PXY, CHIRAL, FIELD, float2, SLAB || FIELD, false>(m, n, nb, w, sid, sn, elecE,
-                                                                                            ld, av, T, invT);
+            res = site_update<POT, FLIP, PRES, CHIRAL, FIELD, float2, false, true>(m, n, nb, w, sid, sn, elecE, ld, av, T,
+                                                                                    invT);
           fin[0] = res.n.x;
           fin[1] = res.n.y;
           fin[2] = res.n.z;
