@@ -85,6 +85,15 @@ __host__ __device__ inline long long dir_index(const RepDesc &r, int c, int x, i
   return r.off + (long long)c * r.comp + ((long long)z * r.py + (y + GY)) * r.px + (x & 1) * r.hp + (x >> 1) + GH;
 }
 
+#ifdef __CUDACC__
+// Programmatic dependent launch: a kernel launched with launch_pdl (launch.h) may start while the kernel before it in
+// the stream ends; it waits here for that kernel's completion and memory, and lets its own successor start early.
+// Nothing the kernels of a sweep write is touched before the wait. The wait ends with the earlier kernel: the hardware
+// starts this one only when every CTA of that one has started.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
+
 // ---- Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11) ------------------------------------------------------
 // Every draw of this library uses a key fixed at compile time per stream and carries the seed in the counter:
 // counter (a, b, seed_lo, seed_hi + c_hi), key (kPhiloxKey0 + stream, kPhiloxKey1). Philox under one key is a

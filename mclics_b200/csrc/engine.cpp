@@ -138,9 +138,10 @@ static void drop_graphs(mcl_engine *e) {
   e->graph_io_series = e->graph_io_stage = nullptr;
 }
 
-// Sweeps per captured graph: one for the in-place colour passes, two for the ping-pong fused kernel (one per
-// buffer parity, so that a replay leaves the buffers where it found them).
-static int graph_sweeps(const mcl_engine *e) { return fused_is_pass_plan(e) ? 1 : 2; }
+// Sweeps per captured graph: eight for the in-place colour passes (kernels overlap at their ends inside a graph, not
+// between two graphs), two for the ping-pong fused kernel (one per buffer parity, so that a replay leaves the buffers
+// where it found them).
+static int graph_sweeps(const mcl_engine *e) { return fused_is_pass_plan(e) ? 8 : 2; }
 
 // Captures graph_sweeps(e) sweeps starting from buffer e->cur as a graph. Every per-sweep quantity the kernels use
 // (sweep counter, temperatures, ang_var, series length) lives in device memory, so a replay does exactly what the

@@ -7,6 +7,7 @@
 #include "launch.h"
 #include "physics.cuh"
 #include "site_access.cuh"
+#include "sweep_draws.cuh"
 
 namespace mcl {
 
@@ -116,6 +117,16 @@ __global__ void __launch_bounds__(kThreads) k_observe(ModelDev m, const RepDesc 
 }
 
 // ------------------------------------------------------------------------------------------------------------
+// S and director of one record.
+__device__ __forceinline__ void solve_record(ObsRecord *r) {
+  double q[6], vec[3];
+#pragma unroll
+  for (int k = 0; k < 6; k++) q[k] = r->q[k];
+  r->S = largest_eigen3(q, vec);
+#pragma unroll
+  for (int k = 0; k < 3; k++) r->director[k] = vec[k];
+}
+
 // One block per replica: deterministic reduction of the replica's partials, ang_var adaptation
 // (src/evolve.cpp:211-220; skipped when adapt = 0), optional series record, reset of the acceptance counter. A
 // series record is left without S and director, which nothing in the sweep loop reads: the serial FP64 Jacobi solve
@@ -131,80 +142,75 @@ __global__ void __launch_bounds__(kThreads) k_finalize(const RepDesc *__restrict
                                                        unsigned long long *__restrict__ sweep_ctr,
                                                        unsigned int *__restrict__ done_ctr, int n_replicas,
                                                        int adapt, const double *__restrict__ gsums) {
-  const int rep = blockIdx.x;
+  const int rep = blockIdx.x, tid = threadIdx.x;
   __shared__ double red[kThreads / 32][kPartials];
-  __shared__ double tot[kPartials];
+  pdl_trigger();
+  const double nv = reps[rep].n_valid;
+  const int b0 = obs_first[rep], b1 = obs_first[rep + 1];
+  pdl_wait();
   const unsigned long long sweep = *sweep_ctr;
   const int slen = *series_len;
-  if (measure && gsums) {
-    if (threadIdx.x < kPartials) tot[threadIdx.x] = gsums[(long long)rep * kZslabSums + threadIdx.x];
-    __syncthreads();
-  } else if (measure) {
-    double acc[kPartials];
-#pragma unroll
-    for (int k = 0; k < kPartials; k++) acc[k] = 0.0;
-    // unrolled: the loads of several items are in flight together (the sums' order does not change)
-#pragma unroll 4
-    for (int b = obs_first[rep] + threadIdx.x; b < obs_first[rep + 1]; b += kThreads)
-#pragma unroll
-      for (int k = 0; k < kPartials; k++) acc[k] += partials[(long long)b * kPartials + k];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < kPartials; k++) {
-      double v = warp_sum_d(acc[k]);
-      if (lane == 0) red[warp][k] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < kPartials) {
-      double v = 0.0;
-      for (int w = 0; w < kThreads / 32; w++) v += red[w][threadIdx.x];
-      tot[threadIdx.x] = v;
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    const RepDesc R = reps[rep];
-    const RepState S = st[rep];
-    const double nv = R.n_valid;
-    const bool probe = measure == 2;  // measurement of the current state only: no adaptation, no counters
-    double a = S.pad;
-    float av = S.ang_var;
+  const RepState S = st[rep];
+  const bool probe = measure == 2;  // measurement of the current state only: no adaptation, no counters
+  // Amplitude and acceptance, which every thread works out (thread 0 stores them).
+  double a = S.pad;
+  float av = S.ang_var;
+  if (!probe) {
     const double nacc = gsums ? gsums[(long long)rep * kZslabSums + kPartials] : (double)S.acc;
-    if (!probe) {
-      a = nacc / nv;
-      if (!adapt) {
-      } else if (1.0 * nacc / nv < 0.5) {
-        av = (float)((double)av * 0.99);
-        if (av < 0.01) av = 0.01f;
-      } else if (1.0 * nacc / nv > 0.5) {
-        av = (float)((double)av / 0.99);
-        if (av > 1.0) av -= 0.5f;
-      }
-      st[rep].ang_var = av;
-      st[rep].pad = (float)a;
-      st[rep].acc = 0ull;
+    a = nacc / nv;
+    if (!adapt) {
+    } else if (1.0 * nacc / nv < 0.5) {
+      av = (float)((double)av * 0.99);
+      if (av < 0.01) av = 0.01f;
+    } else if (1.0 * nacc / nv > 0.5) {
+      av = (float)((double)av / 0.99);
+      if (av > 1.0) av -= 0.5f;
     }
-    if (measure) {
-      ObsRecord o;
-      o.energy = tot[0] / nv;
-      for (int k = 0; k < 6; k++) o.q[k] = tot[1 + k] / nv;
-      if (probe) o.S = largest_eigen3(o.q, o.director);
-      for (int k = 0; k < 3; k++) o.nsum[k] = tot[7 + k];
-      o.n_valid = nv;
-      o.acceptance = a;
-      o.ang_var = av;
-      o.sweep = (double)sweep;
-      series[(long long)slen * n_replicas + rep] = o;
+  }
+  ObsRecord *o = series + (long long)slen * n_replicas + rep;
+  if (measure) {
+    double v = 0.0;  // total of partial tid
+    if (gsums) {
+      if (tid < kPartials) v = gsums[(long long)rep * kZslabSums + tid];
+    } else {
+      double acc[kPartials], mine;
+#pragma unroll
+      for (int k = 0; k < kPartials; k++) acc[k] = 0.0;
+      // unrolled: the loads of several items are in flight together (the sums' order does not change)
+#pragma unroll 4
+      for (int b = b0 + tid; b < b1; b += kThreads)
+#pragma unroll
+        for (int k = 0; k < kPartials; k++) acc[k] += partials[(long long)b * kPartials + k];
+      const int k = warp_sum10(acc, mine);
+      if (k >= 0) red[tid >> 5][k] = mine;
+      __syncthreads();
+      if (tid < kPartials)
+        for (int w = 0; w < kThreads / 32; w++) v += red[w][tid];
     }
-    if (!probe) {
+    // one field per thread (the quotients of a serial tail would follow one another)
+    if (tid == 0) o->energy = v / nv;
+    else if (tid <= 6) o->q[tid - 1] = v / nv;
+    else if (tid < kPartials) o->nsum[tid - 7] = v;
+    else if (tid == 10) o->n_valid = nv;
+    else if (tid == 11) o->acceptance = a;
+    else if (tid == 12) o->ang_var = av;
+    else if (tid == 13) o->sweep = (double)sweep;
+    if (probe) {
+      __syncthreads();
+      if (tid == 0) solve_record(o);
+    }
+  }
+  if (tid == 0 && !probe) {
+    st[rep].ang_var = av;
+    st[rep].pad = (float)a;
+    st[rep].acc = 0ull;
+    __threadfence();
+    const unsigned prev = atomicAdd(done_ctr, 1u);
+    if (prev == (unsigned)gridDim.x - 1) {
+      *done_ctr = 0u;
+      *sweep_ctr = sweep + 1ull;
+      if (measure) *series_len = slen + 1;
       __threadfence();
-      const unsigned prev = atomicAdd(done_ctr, 1u);
-      if (prev == (unsigned)gridDim.x - 1) {
-        *done_ctr = 0u;
-        *sweep_ctr = sweep + 1ull;
-        if (measure) *series_len = slen + 1;
-        __threadfence();
-      }
     }
   }
 }
@@ -344,15 +350,6 @@ cudaError_t launch_observe(const LaunchCtx &c, int geo, const BlockTable &sites,
 }
 
 // S and director of `count` consecutive series records, one thread each.
-__device__ __forceinline__ void solve_record(ObsRecord *r) {
-  double q[6], vec[3];
-#pragma unroll
-  for (int k = 0; k < 6; k++) q[k] = r->q[k];
-  r->S = largest_eigen3(q, vec);
-#pragma unroll
-  for (int k = 0; k < 3; k++) r->director[k] = vec[k];
-}
-
 __global__ void __launch_bounds__(32) k_series_eigen(ObsRecord *__restrict__ series, long long first, long long count) {
   const long long i = (long long)blockIdx.x * 32 + threadIdx.x;
   if (i < count) solve_record(series + first + i);
@@ -365,10 +362,8 @@ cudaError_t launch_series_eigen(cudaStream_t stream, ObsRecord *series, long lon
 
 cudaError_t launch_finalize(const LaunchCtx &c, const BlockTable &sites, const double *partials, int measure,
                             ObsRecord *series, int *series_len, unsigned int *done_ctr, const double *gsums) {
-  k_finalize<<<c.n_replicas, kThreads, 0, c.stream>>>(c.reps, c.state, sites.first, partials, measure, series,
-                                                       series_len, c.sweep_ctr, done_ctr, c.n_replicas, c.adapt,
-                                                       gsums);
-  return cudaGetLastError();
+  return launch_pdl(k_finalize, c.n_replicas, kThreads, 0, c.stream, c.reps, c.state, sites.first, partials, measure,
+                    series, series_len, c.sweep_ctr, done_ctr, c.n_replicas, c.adapt, gsums);
 }
 
 // One block per replica: the replica's partials summed over its blocks (the order k_finalize uses; zeros when

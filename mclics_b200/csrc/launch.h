@@ -34,6 +34,25 @@ struct LaunchCtx {
 
 constexpr int kThreads = 256;
 
+#ifdef __CUDACC__
+// Launch of a kernel that begins with pdl_wait (common.cuh): it may overlap the end of the kernel before it. A sweep is
+// three short dependent kernels; without this each one's launch and first loads follow the last CTA of the one before.
+template <typename... P, typename... A>
+cudaError_t launch_pdl(void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, A &&...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
+}
+#endif
+
 // One sweep with the two-colour schedule, one thread per site and colour (in place).
 cudaError_t launch_sweep_checker2_simple(const LaunchCtx &c, int geo, const BlockTable &half);
 // One sweep in the reference CPU order (8 sublattices, i fastest) with the reference arithmetic (in place).

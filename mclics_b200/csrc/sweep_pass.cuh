@@ -45,6 +45,7 @@
 #pragma once
 #include <type_traits>
 
+#include "launch.h"
 #include "sweep_draws.cuh"
 #include "sweep_fused.cuh"
 
@@ -116,9 +117,9 @@ __global__ void __launch_bounds__(NT, MINB) k_sweep_pass(ModelDev m, FusedArgs a
   float *slots = reinterpret_cast<float *>(smem_raw);
   unsigned long long *bars = reinterpret_cast<unsigned long long *>(smem_raw + (size_t)NSLP * SLOT * 4);
   __shared__ int s_fail;
+  pdl_trigger();
   const FusedItem it = a.items[blockIdx.x];
   const RepDesc R = a.reps[it.rep];
-  const RepState S = a.st[it.rep];
   const int tid = threadIdx.x;
   const CUtensorMap *map = a.tmaps + 2 * it.rep + a.cur;
   const int nx = R.nx, ny = R.ny, nz = R.nz;
@@ -127,17 +128,18 @@ __global__ void __launch_bounds__(NT, MINB) k_sweep_pass(ModelDev m, FusedArgs a
   const int j0 = x0 >> 1;
   const int colour = a.colour;
   constexpr bool measure = MEAS;  // the colour-1 pass with the observables (a.measure != 0, colour 1)
-  const unsigned long long seed = R.seed, sweep = *a.sweep_ctr;
-  const float T = S.T, invT = 1.f / S.T, av = S.ang_var, elecE = S.elecE;
-  constexpr unsigned box_bytes = 3u * PF * 4u;
-
   if (tid == 0) {
     s_fail = 0;
     for (int q = 0; q < NSLP; q++) mbar_init(&bars[q], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
   }
+  pdl_wait();  // the items, layouts and tensor maps above are not written by any sweep; all that follows may be
   __syncthreads();
+  const RepState S = a.st[it.rep];
+  const unsigned long long seed = R.seed, sweep = *a.sweep_ctr;
+  const float T = S.T, invT = 1.f / S.T, av = S.ang_var, elecE = S.elecE;
+  constexpr unsigned box_bytes = 3u * PF * 4u;
 
   // Planes z0 - 1 .. z1 stream through the NSLP slots (plane p in slot (p - pbeg) % NSLP).
   const int pbeg = z0 - 1, pend = z1;
@@ -445,11 +447,7 @@ cudaError_t launch_pass_one(const ModelDev &m, const FusedArgs &a, const FusedLa
     const cudaError_t e = cudaFuncSetAttribute(k0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem);
     return e != cudaSuccess ? e : cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem);
   }
-  if (a.measure != 0 && a.colour == 1)
-    k1<<<l.n_items, NT, l.smem, l.stream>>>(m, a);
-  else
-    k0<<<l.n_items, NT, l.smem, l.stream>>>(m, a);
-  return cudaGetLastError();
+  return launch_pdl(a.measure != 0 && a.colour == 1 ? k1 : k0, l.n_items, NT, l.smem, l.stream, m, a);
 }
 
 // Colour-pass tile configurations (numbering continues the fused kernel's): 2: 64 x 16, 256 threads, 3 CTAs/SM;
