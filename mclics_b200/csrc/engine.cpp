@@ -53,9 +53,9 @@ static void lab_axis(float theta_deg, float phi_deg, float out[3]) {
 // r < nz/2 - 1, one surface layer (radial normal) for r < nz/2 + 1, empty outside.
 static void sphere_geometry(int nx, int ny, int nz, int *pt, float *ns) {
   const float Hx = nx / 2, Hy = ny / 2, Hz = nz / 2;
-  for (int i = 0; i < nx; i++)
+  for (int k = 0; k < nz; k++)
     for (int j = 0; j < ny; j++)
-      for (int k = 0; k < nz; k++) {
+      for (int i = 0; i < nx; i++) {
         const long long idx = i + (long long)nx * (j + (long long)ny * k);
         float Rx = i - Hx, Ry = j - Hy, Rz = k - Hz;
         float radius = sqrt(Rx * Rx + Ry * Ry + Rz * Rz);
@@ -101,6 +101,80 @@ static void free_table(BlockTable &t) {
   cudaFree(t.base);
   cudaFree(t.first);
   t = BlockTable();
+}
+
+static void free_pt_lists(PtLists &t) {
+  cudaFree(t.blocks);
+  cudaFree(t.sites);
+  cudaFree(t.first);
+  t = PtLists();
+}
+
+// The site lists of the point-type sweep from the engine's point types. If the device has no room for them, the engine
+// goes on with the kernel that needs none (no list: n_blocks = 0).
+static int build_pt_lists(mcl_engine *e) {
+  CK(cudaStreamSynchronize(e->stream));
+  free_pt_lists(e->pt_lists);
+  e->pt_lists_stale = false;
+  std::vector<PtSite> sites;
+  std::vector<PtBlock> blocks;
+  std::vector<int> first;
+  std::vector<PtSite> other;  // colour 1 of the replica at hand
+  for (int r = 0; r < e->n_rep; r++) {
+    const RepDesc &D = e->desc[r];
+    const int *pt = e->host_pt.data() + D.site_off;
+    const long long sx = 1, sy = D.nx, sz = (long long)D.nx * D.ny;
+    const size_t begin = sites.size();
+    other.clear();
+    for (int z = 0; z < D.nz; z++)
+      for (int y = 0; y < D.ny; y++) {
+        const long long row = y * sy + z * sz;
+        // steps to the neighbours along y and z (0: no neighbour on this side)
+        const long long yp = y + 1 < D.ny ? sy : (D.periodic[1] ? -(D.ny - 1) * sy : 0);
+        const long long ym = y > 0 ? -sy : (D.periodic[1] ? (D.ny - 1) * sy : 0);
+        const long long zp = z + 1 < D.nz ? sz : (D.periodic[2] ? -(D.nz - 1) * sz : 0);
+        const long long zm = z > 0 ? -sz : (D.periodic[2] ? (D.nz - 1) * sz : 0);
+        for (int x = 0; x < D.nx; x++) {
+          const long long q = row + x;
+          if (pt[q] == 0) continue;
+          const long long xp = x + 1 < D.nx ? sx : (D.periodic[0] ? -(D.nx - 1) * sx : 0);
+          const long long xm = x > 0 ? -sx : (D.periodic[0] ? (D.nx - 1) * sx : 0);
+          const long long step[6] = {xp, xm, yp, ym, zp, zm};
+          uint32_t flags = (uint32_t)pt[q] << 8;
+          for (int d = 0; d < 6; d++)
+            if (step[d] != 0 && pt[q + step[d]] != 0) flags |= 1u << d;
+          (((x + y + z) & 1) ? other : sites).push_back(PtSite{(uint32_t)q, flags});
+        }
+      }
+    const long long n0 = (long long)(sites.size() - begin), n1 = (long long)other.size();
+    sites.insert(sites.end(), other.begin(), other.end());
+    first.push_back((int)blocks.size());
+    for (long long b = 0; b < std::max(n0, n1); b += kPtBlock) {
+      PtBlock B{};
+      B.rep = r;
+      B.count[0] = (int)std::max<long long>(0, std::min<long long>(kPtBlock, n0 - b));
+      B.count[1] = (int)std::max<long long>(0, std::min<long long>(kPtBlock, n1 - b));
+      B.first[0] = (long long)begin + b;
+      B.first[1] = (long long)begin + n0 + b;
+      blocks.push_back(B);
+    }
+  }
+  first.push_back((int)blocks.size());
+  // one row of partials per block, in the engine's buffer (a block per 256 sites of the box)
+  if (blocks.empty() || (long long)blocks.size() > (long long)e->sites.n_blocks) return MCL_OK;
+  PtLists &t = e->pt_lists;
+  if (cudaMalloc(&t.sites, sites.size() * sizeof(PtSite)) != cudaSuccess ||
+      cudaMalloc(&t.blocks, blocks.size() * sizeof(PtBlock)) != cudaSuccess ||
+      cudaMalloc(&t.first, first.size() * sizeof(int)) != cudaSuccess) {
+    cudaGetLastError();
+    free_pt_lists(t);
+    return MCL_OK;
+  }
+  CK(cudaMemcpy(t.sites, sites.data(), sites.size() * sizeof(PtSite), cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(t.blocks, blocks.data(), blocks.size() * sizeof(PtBlock), cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(t.first, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice));
+  t.n_blocks = (int)blocks.size();
+  return MCL_OK;
 }
 
 static int ensure_series(mcl_engine *e, int rows) {
@@ -395,6 +469,8 @@ int mcl_create(const mcl_model *model, const mcl_replica *replicas, int n_replic
   if (schedule == MCL_SCHED_CHECKER2 && fused_supported(e)) {
     if ((rc = fused_create(e)) != MCL_OK) return cleanup_fail(rc);
   }
+  if (geo_class == GEO_PT && e->geometry_set && schedule == MCL_SCHED_CHECKER2 && (rc = build_pt_lists(e)) != MCL_OK)
+    return cleanup_fail(rc);
   e->ghosts_dirty = true;
   if ((rc = refresh_ghosts(e)) != MCL_OK) return cleanup_fail(rc);
   CKC(cudaStreamSynchronize(e->stream));
@@ -411,6 +487,7 @@ int mcl_destroy(mcl_engine *e) {
   free_table(e->half);
   free_table(e->boxes);
   free_table(e->sites);
+  free_pt_lists(e->pt_lists);
   cudaFree(e->d_dir[0]);
   cudaFree(e->d_dir[1]);
   cudaFree(e->d_mlp);
@@ -467,6 +544,7 @@ int mcl_set_geometry(mcl_engine *e, int replica, const int *pt, const float *nor
   CK(cudaMemcpyAsync(e->d_desc + replica, &e->desc[replica], sizeof(RepDesc), cudaMemcpyHostToDevice, e->stream));
   CK(cudaStreamSynchronize(e->stream));
   e->geometry_set = true;
+  e->pt_lists_stale = true;
   return MCL_OK;
 }
 
@@ -631,6 +709,7 @@ static int sweeps_run(mcl_engine *e, int n, int measure) {
   if (measure && (rc = ensure_series(e, e->series_len + n))) return rc;
   const bool use_fused = e->fused && !e->record_dec && !e->d_mlp;
   if (use_fused && (rc = refresh_ghosts(e))) return rc;
+  if (e->geo == GEO_PT && e->pt_lists_stale && e->schedule == MCL_SCHED_CHECKER2 && (rc = build_pt_lists(e))) return rc;
   if (use_fused && fused_resident(e)) {
     // one launch for up to kResidentSweeps sweeps (bounded, so that a long call leaves the device now and then)
     constexpr int kResidentSweeps = 1024;
@@ -696,7 +775,20 @@ static int sweeps_run(mcl_engine *e, int n, int measure) {
         e->ghosts_dirty = true;
         if (measure) e->series_len++;
         continue;
-      } else if (e->schedule == MCL_SCHED_REF8) {
+      }
+      if (e->pt_lists.n_blocks && e->schedule == MCL_SCHED_CHECKER2 && !e->record_dec) {  // point types, by site lists
+        CK(launch_sweep_pt(c, e->pt_lists, measure ? 1 : 0, e->d_partials));
+        e->launches += 2;
+        if (ev1) CK(cudaEventRecord(ev1, e->stream));
+        BlockTable t;
+        t.first = e->pt_lists.first;
+        CK(launch_finalize(c, t, e->d_partials, measure ? 1 : 0, e->d_series, e->d_series_len, e->d_done));
+        e->launches++;
+        e->ghosts_dirty = true;
+        if (measure) e->series_len++;
+        continue;
+      }
+      if (e->schedule == MCL_SCHED_REF8) {
         CK(launch_sweep_ref8(c, e->geo, e->boxes));
         e->launches += 8;
       } else {

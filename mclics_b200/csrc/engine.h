@@ -60,6 +60,8 @@ struct mcl_engine {
   bool geometry_set = true;
 
   mcl::BlockTable half, boxes, sites;
+  mcl::PtLists pt_lists;      // sphere and custom: non-empty sites per colour (built when the geometry is known)
+  bool pt_lists_stale = true;
   std::vector<int> host_pt;  // point types (GEO_PT), for n_valid
   mcl::FusedPlan *fused = nullptr;
   cudaStream_t own_stream = nullptr;

@@ -60,6 +60,141 @@ __global__ void __launch_bounds__(kThreads) k_sweep_color(ModelDev m, const RepD
 }
 
 // ------------------------------------------------------------------------------------------------------------
+// Two-colour sweep of point-type lattices (sphere, custom) over lists of their non-empty sites.
+//
+// k_sweep_color gives every cell of the box a thread: in a droplet 48 % of them are empty, and each of the others spends
+// 64-bit divisions, seven dependent point-type loads and a full general trial on its site, then a measured sweep reads
+// everything again (k_observe). Here a replica and colour have a list of sites with what the geometry says about them
+// (PtSite, built when the geometry is set), so every thread has a site, its neighbours' directors are requested at once,
+// and the kernel is compiled for the model's options. Same draws, same bond form and rounding, so the same decisions.
+// The observables of a measured sweep come with the update, as in the learned sweep: every bond has one colour-1 end, so
+// E = sum_1 (2 bond + single) + sum_0 single.
+//
+// Bound by the latency of one site's chain at small sizes (one wave), by instruction issue above. Sphere 64^3 GHRL with
+// homeotropic anchoring, 50 + 50 sweeps with their series and field: 3774 us before, 1929 us now.
+constexpr int kPtThreads = kPtBlock;
+
+template <int POT, bool FLIP, int CHIRAL, bool FIELD, bool MEAS>
+__global__ void __launch_bounds__(kPtThreads) k_sweep_pt(ModelDev m, const RepDesc *__restrict__ reps, RepState *__restrict__ st,
+                                                         float *__restrict__ dir, const float *__restrict__ nrm,
+                                                         const unsigned long long *__restrict__ sweep_ctr, int colour,
+                                                         const PtBlock *__restrict__ blocks,
+                                                         const PtSite *__restrict__ sites,
+                                                         double *__restrict__ partials) {
+  pdl_trigger();
+  const PtBlock B = blocks[blockIdx.x];
+  const RepDesc &R = reps[B.rep];
+  const bool valid = (int)threadIdx.x < B.count[colour];
+  PtSite site{0, 0};
+  if (valid) site = sites[B.first[colour] + threadIdx.x];
+  const unsigned nx = (unsigned)R.nx, ny = (unsigned)R.ny, row = site.q / nx;
+  const int x = (int)(site.q - row * nx), z = (int)(row / ny), y = (int)(row - (unsigned)z * ny);
+  pdl_wait();
+  unsigned accepted = 0;
+  double acc[kPartials];
+#pragma unroll
+  for (int k = 0; k < kPartials; k++) acc[k] = 0.0;
+  if (valid) {
+    const RepState S = st[B.rep];
+    const long long comp = R.comp, rowp = R.px, planep = (long long)R.py * R.px;
+    const int half_x = (x & 1) * R.hp + (x >> 1);
+    float *c0 = dir + R.off + z * planep + (long long)(y + GY) * rowp + GH + half_x;
+    auto load = [&](const float *q) { return Vec3{q[0], q[comp], q[2 * comp]}; };
+    const Vec3 n = load(c0);
+    Vec3 nb[6];
+    float w[6];
+#pragma unroll
+    for (int d = 0; d < 6; d++) {
+      const int axis = d >> 1, delta = (d & 1) ? -1 : 1;
+      long long off;  // of the neighbour's cell, wrapped along a periodic axis
+      if (axis == 0) {
+        int v = x + delta;
+        v = v < 0 ? v + R.nx : (v >= R.nx ? v - R.nx : v);
+        off = (v & 1) * R.hp + (v >> 1) - half_x;
+      } else if (axis == 1) {
+        off = (y + delta < 0 ? R.ny - 1 : (y + delta >= R.ny ? 1 - R.ny : delta)) * rowp;
+      } else {
+        off = (z + delta < 0 ? R.nz - 1 : (z + delta >= R.nz ? 1 - R.nz : delta)) * planep;
+      }
+      const bool there = (site.flags >> d) & 1u;
+      nb[d] = there ? load(c0 + off) : Vec3{0.f, 0.f, 0.f};
+      w[d] = there ? 1.f : 0.f;
+    }
+    const int sid = (int)(site.flags >> 8) - 2;  // point type 1: bulk
+    Vec3 s{0.f, 0.f, 0.f};
+    if (sid >= 0) {
+      const float *v = nrm + 3 * (R.site_off + site.q);
+      s = Vec3{v[0], v[1], v[2]};
+    }
+    const LaneDraw<float> ld = lane_draw(site_draw(R.seed, *sweep_ctr, x, y, z, nx, ny, FLIP), FLIP);
+    const SiteResultT<float> r = site_update<POT, FLIP, 0, CHIRAL, FIELD, float>(m, n, nb, w, sid, s, S.elecE, ld,
+                                                                                S.ang_var, S.T, 1.f / S.T);
+    accepted = r.rot ? 1u : 0u;
+    if (r.rot || r.flip) {
+      c0[0] = r.n.x;
+      c0[comp] = r.n.y;
+      c0[2 * comp] = r.n.z;
+    }
+    if (MEAS) {
+      acc[0] = (double)(colour == 0 ? r.single : __fadd_rn(__fmul_rn(2.f, r.bond), r.single));
+      const double dx = r.n.x, dy = r.n.y, dz = r.n.z;
+      acc[1] = 1.5 * dx * dx - 0.5;
+      acc[2] = 1.5 * dx * dy;
+      acc[3] = 1.5 * dx * dz;
+      acc[4] = 1.5 * dy * dy - 0.5;
+      acc[5] = 1.5 * dy * dz;
+      acc[6] = 1.5 * dz * dz - 0.5;
+      acc[7] = dx;
+      acc[8] = dy;
+      acc[9] = dz;
+    }
+  }
+  const unsigned wsum = __reduce_add_sync(0xffffffffu, accepted);
+  if ((threadIdx.x & 31) == 0 && wsum) atomicAdd(&st[B.rep].acc, (unsigned long long)wsum);
+  if (MEAS) {
+    __shared__ double red[kPtThreads / 32][kPartials];
+    double mine;
+    const int k = warp_sum10(acc, mine);
+    if (k >= 0) red[threadIdx.x >> 5][k] = mine;
+    __syncthreads();
+    if (threadIdx.x < kPartials) {
+      double v = 0.0;
+      for (int w2 = 0; w2 < kPtThreads / 32; w2++) v += red[w2][threadIdx.x];
+      double *dst = partials + (long long)blockIdx.x * kPartials + threadIdx.x;
+      *dst = colour == 0 ? v : *dst + v;
+    }
+  }
+}
+
+template <int POT, bool FLIP, int CHIRAL, bool FIELD>
+static cudaError_t sweep_pt_one(const LaunchCtx &c, const PtLists &t, int measure, double *partials) {
+  for (int colour = 0; colour < 2; colour++) {
+    const cudaError_t e = launch_pdl(measure ? k_sweep_pt<POT, FLIP, CHIRAL, FIELD, true> : k_sweep_pt<POT, FLIP, CHIRAL, FIELD, false>,
+                                     t.n_blocks, kPtThreads, 0, c.stream, c.model, c.reps, c.state, c.dir, c.nrm,
+                                     c.sweep_ctr, colour, t.blocks, t.sites, partials);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+template <int POT, int CHIRAL>
+static cudaError_t sweep_pt_pot(const LaunchCtx &c, const PtLists &t, int measure, double *partials) {
+  if (c.model.flip)
+    return c.model.field_on ? sweep_pt_one<POT, true, CHIRAL, true>(c, t, measure, partials)
+                            : sweep_pt_one<POT, true, CHIRAL, false>(c, t, measure, partials);
+  return c.model.field_on ? sweep_pt_one<POT, false, CHIRAL, true>(c, t, measure, partials)
+                          : sweep_pt_one<POT, false, CHIRAL, false>(c, t, measure, partials);
+}
+
+cudaError_t launch_sweep_pt(const LaunchCtx &c, const PtLists &t, int measure, double *partials) {
+  if (c.model.potential == POT_GHRL)
+    return c.model.sigma != 0.f ? sweep_pt_pot<POT_GHRL, 1>(c, t, measure, partials)
+                                : sweep_pt_pot<POT_GHRL, 2>(c, t, measure, partials);
+  if (c.model.potential == POT_PEAR) return sweep_pt_pot<POT_PEAR, 2>(c, t, measure, partials);
+  return sweep_pt_pot<POT_LL, 2>(c, t, measure, partials);
+}
+
+// ------------------------------------------------------------------------------------------------------------
 // Observables of the current state: per block sums of the site energies, (3 n n - I)/2 and n, in FP64.
 __device__ __forceinline__ double warp_sum_d(double v) {
 #pragma unroll

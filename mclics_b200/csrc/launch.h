@@ -18,6 +18,25 @@ struct BlockTable {
   int *first = nullptr;       // device, n_replicas + 1 entries: first block of each replica
 };
 
+// Site lists of point-type replicas (k_sweep_pt): per replica and colour the non-empty sites in linear order. Block b of
+// a launch takes entries first[colour] .. first[colour] + count[colour] - 1 of replica rep.
+struct PtSite {
+  uint32_t q;      // linear index in the replica
+  uint32_t flags;  // bits 0-5: neighbours present (+x, -x, +y, -y, +z, -z); bits 8 up: point type
+};
+struct PtBlock {
+  int rep;
+  int count[2];
+  int pad;
+  long long first[2];
+};
+struct PtLists {
+  int n_blocks = 0;
+  PtBlock *blocks = nullptr;  // device
+  PtSite *sites = nullptr;    // device
+  int *first = nullptr;       // device, n_replicas + 1 entries: first block of each replica
+};
+
 struct LaunchCtx {
   ModelDev model;
   int n_replicas;
@@ -55,6 +74,10 @@ cudaError_t launch_pdl(void (*k)(P...), unsigned grid, unsigned block, size_t sm
 
 // One sweep with the two-colour schedule, one thread per site and colour (in place).
 cudaError_t launch_sweep_checker2_simple(const LaunchCtx &c, int geo, const BlockTable &half);
+// One sweep with the two-colour schedule over the site lists of point-type replicas; with measure, the observables of
+// the final state go to partials[block][kPartials].
+cudaError_t launch_sweep_pt(const LaunchCtx &c, const PtLists &t, int measure, double *partials);
+constexpr int kPtBlock = 128;  // sites per block of a list
 // One sweep in the reference CPU order (8 sublattices, i fastest) with the reference arithmetic (in place).
 cudaError_t launch_sweep_ref8(const LaunchCtx &c, int geo, const BlockTable &boxes);
 // Observables of the current state into partials[block][kPartials].

@@ -89,9 +89,10 @@ __device__ __forceinline__ L ll_bond(const ModelDev &m, const V3<L> &x, const V3
   return mul_(splat<L>(-1.5f * m.A), mul_(b, b));
 }
 
-// GHRL with bond vector r = sign * e_axis, src/potential.cpp:40-56. CHIRAL = false drops the sigma term, which
-// is exact for sigma = 0 (fma(0, c, u) == u).
-template <int AXIS, bool CHIRAL, typename L>
+// GHRL with bond vector r = sign * e_axis, src/potential.cpp:40-56. Only CHIRAL = 1 has the sigma term, whose absence
+// is exact for sigma = 0 (fma(0, c, u) == u). CHIRAL = 2 selects this bond form without it; CHIRAL = 0 the site sums of
+// ghrl_sums, which round differently.
+template <int AXIS, int CHIRAL, typename L>
 __device__ __forceinline__ L ghrl_bond(const ModelDev &m, const V3<L> &x, const V3<L> &y, float sign) {
   const L ai = comp<AXIS>(x), aj = comp<AXIS>(y);  // a_i a_j and a^2 do not depend on the sign of r
   const L b = dot(x, y);
@@ -99,7 +100,7 @@ __device__ __forceinline__ L ghrl_bond(const ModelDev &m, const V3<L> &x, const 
   const L e1 = fma_(splat<L>(1.5f), fma_(ai, ai, mul_(aj, aj)), splat<L>(-1.f));
   L u = fma_(e1, fma_(splat<L>(m.rho), p2, splat<L>(m.lam)),
              fma_(splat<L>(m.mu), fma_(mul_(ai, aj), b, splat<L>(-1.f / 9.f)), mul_(splat<L>(m.nu), p2)));
-  if (CHIRAL) {
+  if (CHIRAL == 1) {
     // c = r . (n_j x n_i)
     const L c = AXIS == 0 ? fma_(y.y, x.z, neg_(mul_(y.z, x.y)))
                           : (AXIS == 1 ? fma_(y.z, x.x, neg_(mul_(y.x, x.z))) : fma_(y.x, x.y, neg_(mul_(y.y, x.x))));
@@ -132,7 +133,7 @@ __device__ __forceinline__ L pear_bond(const ModelDev &m, const V3<L> &x, const 
   return fma_(mul_(splat<L>(-m.A), b), b, fma_(splat<L>(-m.B1), b, mul_(splat<L>(-0.25f * m.C), ps)));
 }
 
-template <int POT, int D, bool CHIRAL, typename L>
+template <int POT, int D, int CHIRAL, typename L>
 __device__ __forceinline__ L bond(const ModelDev &m, const V3<L> &x, const V3<L> &y) {
   if (POT == POT_LL) return ll_bond(m, x, y);
   if (POT == POT_GHRL) return ghrl_bond<BondDir<D>::axis, CHIRAL>(m, x, y, BondDir<D>::sign);
@@ -144,7 +145,7 @@ __device__ __forceinline__ L bond(const ModelDev &m, const V3<L> &x, const V3<L>
 // kPresentXY those along x and y, kPresentZ those along z. The two-director form evaluates both in one pass, so each neighbour is used once.
 constexpr int kPresentXY = 1, kPresentZ = 2;
 __host__ __device__ constexpr bool present(int pres, int d) { return (pres & (d < 4 ? kPresentXY : kPresentZ)) != 0; }
-template <int POT, int PRES, bool CHIRAL, int D, typename L>
+template <int POT, int PRES, int CHIRAL, int D, typename L>
 __device__ __forceinline__ L acc_bond(const ModelDev &m, const V3<L> &x, const V3<L> &y, const L &w, const L &e) {
   const L u = bond<POT, D, CHIRAL>(m, x, y);
   if (present(PRES, D)) return D == 0 ? u : add_(e, u);
@@ -225,10 +226,10 @@ __device__ __forceinline__ void ghrl_sums(const ModelDev &m, const V3<L> *const 
   for (int i = 0; i < NS; i++) out[i] = fma_(splat<L>(1.5f * m.nu), sB[i], add_(e[i], c));
 }
 
-template <int POT, int PRES, bool CHIRAL, typename L>
+template <int POT, int PRES, int CHIRAL, typename L>
 __device__ __forceinline__ L bond_sum(const ModelDev &m, const V3<L> &x, const V3<L> (&nb)[6], const L (&w)[6]) {
   if (POT == POT_LL) return ll_sum<PRES>(m, x, nb, w);
-  if (POT == POT_GHRL && !CHIRAL) {
+  if (POT == POT_GHRL && CHIRAL == 0) {
     const V3<L> *const xs[1] = {&x};
     L out[1];
     ghrl_sums<PRES, 1>(m, xs, nb, w, out);
@@ -243,7 +244,7 @@ __device__ __forceinline__ L bond_sum(const ModelDev &m, const V3<L> &x, const V
   return e;
 }
 
-template <int POT, int PRES, bool CHIRAL, typename L>
+template <int POT, int PRES, int CHIRAL, typename L>
 __device__ __forceinline__ void bond_sum2(const ModelDev &m, const V3<L> &x, const V3<L> &x2, const V3<L> (&nb)[6],
                                           const L (&w)[6], L &e1, L &e2) {
   if (POT == POT_LL) {
@@ -262,7 +263,7 @@ __device__ __forceinline__ void bond_sum2(const ModelDev &m, const V3<L> &x, con
     e2 = mul_(splat<L>(-1.5f * m.A), s2);
     return;
   }
-  if (POT == POT_GHRL && !CHIRAL) {
+  if (POT == POT_GHRL && CHIRAL == 0) {
     const V3<L> *const xs[2] = {&x, &x2};
     L out[2];
     ghrl_sums<PRES, 2>(m, xs, nb, w, out);
@@ -451,7 +452,7 @@ __device__ __forceinline__ V3<L> sel3(LB<L> c, const V3<L> &a, const V3<L> &b) {
 // FIELD (field term), SINGLE = false (the caller knows the site has no single-site term: no surface, no field;
 // the energies are then the bond sums themselves, which is what adding the zero single term gives, up to the sign
 // of a zero). Every combination rounds like the general one on the inputs it applies to.
-template <int POT, bool FLIP, int PRES, bool CHIRAL, bool FIELD, typename L, bool SINGLE = true, bool FUSED = false>
+template <int POT, bool FLIP, int PRES, int CHIRAL, bool FIELD, typename L, bool SINGLE = true, bool FUSED = false>
 __device__ __forceinline__ SiteResultT<L> site_update(const ModelDev &m, const V3<L> &n, const V3<L> (&nb)[6],
                                                       const L (&w)[6], int sid, const Vec3 &s, float elecE,
                                                       const LaneDraw<L> &d, float av, float T, float invT) {
