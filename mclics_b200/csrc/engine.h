@@ -9,11 +9,15 @@
 #include "common.cuh"
 #include "launch.h"
 
+struct mcl_engine;
+
 namespace mcl {
 
 // Sets the thread's last error message and returns code.
 int fail(int code, const char *fmt, ...);
 int cuda_fail(cudaError_t err, const char *what);
+// Device memory to a caller's pageable memory on the engine's stream; returns when it has arrived.
+int copy_out(mcl_engine *e, void *dst, const void *d_src, size_t bytes);
 
 struct FusedPlan;  // fused tiled sweep (sweep_fused.cu)
 struct MlpDev;     // learned proposal weights in device layout (learned.cu)
@@ -89,6 +93,8 @@ struct mcl_engine {
   const void *graph_series = nullptr;             // series buffer the measuring graph writes
   cudaGraphExec_t graph_io = nullptr;  // mcl_sweeps_io's step (input kernel, one measured sweep, output kernel)
   const void *graph_io_series = nullptr, *graph_io_stage = nullptr;  // the buffers it was captured with
+  char *h_copy = nullptr;    // pinned ring of large device-to-host copies (copy_out), one slot per copying thread
+  std::vector<cudaEvent_t> copy_ev;
   void *h_io = nullptr;      // mapped pinned staging of mcl_sweeps_io: error words, temperatures, observables records
   void *d_io = nullptr;      // its device address
   size_t h_io_bytes = 0;

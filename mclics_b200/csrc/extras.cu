@@ -238,7 +238,5 @@ extern "C" int mcl_local_order(mcl_engine *e, int replica, float *S) {
   }
   CKX(cudaGetLastError());
   e->launches++;
-  CKX(cudaMemcpyAsync(S, out, (size_t)N * sizeof(float), cudaMemcpyDeviceToHost, c.stream));
-  CKX(cudaStreamSynchronize(c.stream));
-  return MCL_OK;
+  return copy_out(e, S, out, (size_t)N * sizeof(float));
 }
