@@ -16,7 +16,7 @@
 //
 // Training (maximum likelihood of the local conditional distribution, loss -log(4 pi q(n | features)) over sites
 // of equilibrated plain-sweep states) runs in FP32 on the CUDA cores with the same BF16 rounding of weights,
-// features and hidden activations as inference: one thread per sample for the forward and backward passes, then
+// features and hidden activations as inference: 64 samples per block, each thread a 4 x 4 tile of every product, then
 // the block's weight gradients from its 64 samples in shared memory, per-block partial sums, and a fixed-order
 // FP64 reduction with the Adam update.
 #include <cuda_bf16.h>
@@ -701,171 +701,207 @@ __global__ void k_extract_samples(const RepDesc *__restrict__ reps, const RepSta
 }
 
 // ---- training ------------------------------------------------------------------------------------------------
-constexpr int kTB = 64;            // samples (threads) per training block
-constexpr int kHP = kH + 1;        // row pitch of the per-sample activation arrays
-constexpr int kWPad = kNP + 4;     // BF16-rounded weights in shared memory
-constexpr size_t kTrainSmem = sizeof(float) * (kWPad + kTB * 9 + 4 * kTB * kHP + kTB * 5 + kTB);
+constexpr int kTB = 64;     // samples per training block
+constexpr int kTT = 256;    // threads per training block: 16 x 16, each a 4 x 4 tile of a 64 x 64 product
+constexpr int kTP = kH + 4;  // row pitch of the tiles in shared memory (rows 16-byte aligned, columns spread over banks)
+struct TrainSmem {
+  float w1[kH * kIn], b1[kH], b2[kH], w3[kOut * kH], b3[kOut];
+  float x[kTB][8], dout[kTB][kOut], loss[kTB];
+  alignas(16) float w2[kH][kTP];    // [out][in]
+  alignas(16) float w2t[kH][kTP];   // [in][out]
+  alignas(16) float h1[kTB][kTP];   // [sample][unit]
+  alignas(16) float h1t[kH][kTP];   // [unit][sample]
+  alignas(16) float h2t[kH][kTP];
+  alignas(16) float dz2[kTB][kTP];
+  alignas(16) float dz2t[kH][kTP];
+  alignas(16) float dz1[kTB][kTP];
+};
+constexpr size_t kTrainSmem = sizeof(TrainSmem);
 
-// Forward and backward pass of kTB samples (one per thread) with the pass copy wr of the parameters; writes this block's
-// parameter gradient of the mean loss (scale = 1 / batch) and its loss sum to partial[blockIdx.x][0 .. kNP].
-__global__ void __launch_bounds__(kTB) k_mlp_grad(const float *__restrict__ wr, const float *__restrict__ feat,
-                                                  const float *__restrict__ dirs, long long n, float kappa_max,
-                                                  float scale, float *__restrict__ partial) {
-  extern __shared__ float sm[];
-  float *W = sm;
-  float *X = W + kWPad;            // [kTB][9]
-  float *H1 = X + kTB * 9;         // [kTB][kHP]
-  float *H2 = H1 + kTB * kHP;
-  float *DZ1 = H2 + kTB * kHP;
-  float *DZ2 = DZ1 + kTB * kHP;
-  float *DO = DZ2 + kTB * kHP;     // [kTB][5]
-  float *LS = DO + kTB * 5;        // [kTB]
-  const int tid = threadIdx.x;
-  for (int i = tid; i < kNP; i += kTB) W[i] = wr[i];
-  __syncthreads();
-  const long long s = (long long)blockIdx.x * kTB + tid;
-  const bool valid = s < n && feat[s * kFeat + 7] != 0.f;
-  float x[kIn];
+// c[u][v] += sum_k a[k][u] b[k][v] over 64 rows k, in order: a thread's 4 x 4 tile of a 64 x 64 product, one 16-byte
+// load of each operand per 16 multiplications.
+__device__ __forceinline__ void tile_product(const float (*a)[kTP], const float (*b)[kTP], int u0, int v0, float (&c)[4][4]) {
+#pragma unroll 8
+  for (int k = 0; k < 64; k++) {
+    const float4 av = *reinterpret_cast<const float4 *>(&a[k][u0]), bv = *reinterpret_cast<const float4 *>(&b[k][v0]);
+    const float au[4] = {av.x, av.y, av.z, av.w}, bb[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
-  for (int k = 0; k < kIn; k++) {
-    x[k] = valid ? bf16r(feat[s * kFeat + k]) : 0.f;
-    X[tid * 9 + k] = x[k];
-  }
-  float z1[kH], h1[kH];
-#pragma unroll 4
-  for (int j = 0; j < kH; j += 2) {
-    float a0 = W[oB1 + j], a1 = W[oB1 + j + 1];
+    for (int u = 0; u < 4; u++)
 #pragma unroll
-    for (int k = 0; k < kIn; k++) {
-      a0 = fmaf(W[oW1 + j * kIn + k], x[k], a0);
-      a1 = fmaf(W[oW1 + (j + 1) * kIn + k], x[k], a1);
-    }
-    z1[j] = a0;
-    z1[j + 1] = a1;
-    const uint32_t hv = silu2(a0, a1);
-    h1[j] = bf_lo(hv);
-    h1[j + 1] = bf_hi(hv);
-    H1[tid * kHP + j] = h1[j];
-    H1[tid * kHP + j + 1] = h1[j + 1];
-  }
-  float z2[kH], h2[kH];
-#pragma unroll 2
-  for (int j = 0; j < kH; j += 2) {
-    float a0 = W[oB2 + j], a1 = W[oB2 + j + 1];
-#pragma unroll
-    for (int i = 0; i < kH; i++) {
-      a0 = fmaf(W[oW2 + j * kH + i], h1[i], a0);
-      a1 = fmaf(W[oW2 + (j + 1) * kH + i], h1[i], a1);
-    }
-    z2[j] = a0;
-    z2[j + 1] = a1;
-    const uint32_t hv = silu2(a0, a1);
-    h2[j] = bf_lo(hv);
-    h2[j + 1] = bf_hi(hv);
-    H2[tid * kHP + j] = h2[j];
-    H2[tid * kHP + j + 1] = h2[j + 1];
-  }
-  float o[kOut];
-#pragma unroll
-  for (int mo = 0; mo < kOut; mo++) {
-    float a = W[oB3 + mo];
-#pragma unroll
-    for (int j = 0; j < kH; j++) a = fmaf(W[oW3 + mo * kH + j], h2[j], a);
-    o[mo] = a;
-  }
-  // head, loss and d loss / d o
-  float dout[kOut] = {0.f, 0.f, 0.f, 0.f};
-  float loss = 0.f;
-  if (valid) {
-    const float nx = dirs[s * 3], ny = dirs[s * 3 + 1], nz = dirs[s * 3 + 2];
-    const float na = sqrtf(fmaf(o[0], o[0], fmaf(o[1], o[1], o[2] * o[2])));
-    const float inv = 1.f / fmaxf(na, 1e-20f);
-    const float mx = o[0] * inv, my = o[1] * inv, mz = o[2] * inv;
-    const float kr = o[3] > 20.f ? o[3] : log1pf(expf(o[3]));
-    const float kappa = fminf(fmaxf(kr, kKappaMin), kappa_max);
-    const float t = fmaf(mx, nx, fmaf(my, ny, mz * nz));
-    const float at = fabsf(t);
-    const float g = kappa * (expf(kappa * (at - 1.f)) + expf(-kappa * (at + 1.f))) / (-expm1f(-2.f * kappa));
-    const float den = fmaf(1.f - kEps, g, kEps);
-    loss = -logf(den);
-    const float th = tanhf(kappa * t);
-    const float dt = -(1.f - kEps) * g * kappa * th / den;
-    const float ikc = kappa < 0.1f ? kappa * (-1.f / 3.f + kappa * kappa / 45.f) : 1.f / kappa - 1.f / tanhf(kappa);
-    float dk = -(1.f - kEps) * g * (ikc + t * th) / den;
-    if (!(kr > kKappaMin && kr < kappa_max)) dk = 0.f;
-    dout[0] = scale * dt * (nx - t * mx) * inv;
-    dout[1] = scale * dt * (ny - t * my) * inv;
-    dout[2] = scale * dt * (nz - t * mz) * inv;
-    dout[3] = scale * dk * sigm_f(o[3]);
-  }
-  LS[tid] = loss;
-#pragma unroll
-  for (int mo = 0; mo < kOut; mo++) DO[tid * 5 + mo] = dout[mo];
-  // backward to the hidden layers (z2 is overwritten with dz2)
-#pragma unroll 4
-  for (int j = 0; j < kH; j++) {
-    float a = 0.f;
-#pragma unroll
-    for (int mo = 0; mo < kOut; mo++) a = fmaf(W[oW3 + mo * kH + j], dout[mo], a);
-    const float sg = sigm_f(z2[j]);
-    z2[j] = a * sg * fmaf(z2[j], 1.f - sg, 1.f);
-    DZ2[tid * kHP + j] = z2[j];
-  }
-#pragma unroll 4
-  for (int i = 0; i < kH; i++) {
-    float a = 0.f;
-#pragma unroll
-    for (int j = 0; j < kH; j++) a = fmaf(W[oW2 + j * kH + i], z2[j], a);
-    const float sg = sigm_f(z1[i]);
-    DZ1[tid * kHP + i] = a * sg * fmaf(z1[i], 1.f - sg, 1.f);
-  }
-  __syncthreads();
-  // this block's weight gradients: thread tid owns column tid of every [out][in] matrix it can
-  float *P = partial + (size_t)blockIdx.x * (kNP + 1);
-  for (int r = 0; r < kH; r++) {  // w2[r][tid] = sum_s dz2[s][r] h1[s][tid]
-    float a = 0.f;
-    for (int q = 0; q < kTB; q++) a = fmaf(DZ2[q * kHP + r], H1[q * kHP + tid], a);
-    P[oW2 + r * kH + tid] = a;
-  }
-  {
-    float a[kIn] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, b1 = 0.f, b2 = 0.f;
-    for (int q = 0; q < kTB; q++) {
-      const float d1 = DZ1[q * kHP + tid];
-#pragma unroll
-      for (int k = 0; k < kIn; k++) a[k] = fmaf(d1, X[q * 9 + k], a[k]);
-      b1 += d1;
-      b2 += DZ2[q * kHP + tid];
-    }
-#pragma unroll
-    for (int k = 0; k < kIn; k++) P[oW1 + tid * kIn + k] = a[k];
-    P[oB1 + tid] = b1;
-    P[oB2 + tid] = b2;
-  }
-#pragma unroll
-  for (int mo = 0; mo < kOut; mo++) {  // w3[mo][tid]
-    float a = 0.f;
-    for (int q = 0; q < kTB; q++) a = fmaf(DO[q * 5 + mo], H2[q * kHP + tid], a);
-    P[oW3 + mo * kH + tid] = a;
-  }
-  if (tid < kOut) {
-    float a = 0.f;
-    for (int q = 0; q < kTB; q++) a += DO[q * 5 + tid];
-    P[oB3 + tid] = a;
-  }
-  if (tid == 0) {
-    float a = 0.f;
-    for (int q = 0; q < kTB; q++) a += LS[q];
-    P[kNP] = a;
+      for (int v = 0; v < 4; v++) c[u][v] = fmaf(au[u], bb[v], c[u][v]);
   }
 }
 
-// Fixed-order FP64 sum of the block partials: gradient (and loss sum in out[kNP]).
-__global__ void k_grad_reduce(const float *__restrict__ partial, int nb, double *__restrict__ out) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p > kNP) return;
-  double a = 0.0;
-  for (int b = 0; b < nb; b++) a += (double)partial[(size_t)b * (kNP + 1) + p];
-  out[p] = a;
+// Forward and backward pass of kTB samples with the pass copy wr of the parameters; writes this block's parameter
+// gradient of the mean loss (scale = 1 / batch) and its loss sum to partial[blockIdx.x][0 .. kNP].
+//
+// Bound by the FP32 pipe in its three 64 x 64 x 64 products (115 M multiply-adds for 8192 samples: 3 us over the chip)
+// and the latency of its phases. One thread per sample, 64 per block, it ran at 3 % of the warps and one shared load per
+// multiplication (55 us); 256 threads with 4 x 4 register tiles take 22 us. Every sum keeps its order of terms, so
+// gradients are the same bits.
+__global__ void __launch_bounds__(kTT) k_mlp_grad(const float *__restrict__ wr, const float *__restrict__ feat,
+                                                  const float *__restrict__ dirs, long long n, float kappa_max,
+                                                  float scale, float *__restrict__ partial) {
+  extern __shared__ __align__(16) unsigned char train_dyn[];
+  TrainSmem &S = *reinterpret_cast<TrainSmem *>(train_dyn);
+  const int tid = threadIdx.x, s0 = 4 * (tid >> 4), j0 = 4 * (tid & 15);  // tile: samples s0 .., units j0 ..
+  pdl_trigger();
+  const long long base = (long long)blockIdx.x * kTB;
+  for (int i = tid; i < kTB * 8; i += kTT) {  // features, rounded to BF16; column 7 the validity flag
+    const long long row = base + (i >> 3);
+    const float f7 = row < n ? feat[row * kFeat + 7] : 0.f;
+    S.x[i >> 3][i & 7] = f7 == 0.f ? 0.f : ((i & 7) == 7 ? 1.f : bf16r(feat[row * kFeat + (i & 7)]));
+  }
+  pdl_wait();  // the parameters are the last step's
+  for (int i = tid; i < kH * kIn; i += kTT) S.w1[i] = wr[oW1 + i];
+  for (int i = tid; i < kH * kH; i += kTT) {
+    const float v = wr[oW2 + i];
+    S.w2[i >> 6][i & 63] = v;
+    S.w2t[i & 63][i >> 6] = v;
+  }
+  for (int i = tid; i < kOut * kH; i += kTT) S.w3[i] = wr[oW3 + i];
+  if (tid < kH) {
+    S.b1[tid] = wr[oB1 + tid];
+    S.b2[tid] = wr[oB2 + tid];
+  }
+  if (tid < kOut) S.b3[tid] = wr[oB3 + tid];
+  __syncthreads();
+  // layer 1 of the tile: z1[sample][unit]
+  float z1[4][4], z2[4][4];
+#pragma unroll
+  for (int u = 0; u < 4; u++) {
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+      float a = S.b1[j0 + v];
+#pragma unroll
+      for (int k = 0; k < kIn; k++) a = fmaf(S.w1[(j0 + v) * kIn + k], S.x[s0 + u][k], a);
+      z1[u][v] = a;
+    }
+#pragma unroll
+    for (int v = 0; v < 4; v += 2) {
+      const uint32_t hv = silu2(z1[u][v], z1[u][v + 1]);
+      S.h1[s0 + u][j0 + v] = S.h1t[j0 + v][s0 + u] = bf_lo(hv);
+      S.h1[s0 + u][j0 + v + 1] = S.h1t[j0 + v + 1][s0 + u] = bf_hi(hv);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < 4; u++)
+#pragma unroll
+    for (int v = 0; v < 4; v++) z2[u][v] = S.b2[j0 + v];
+  tile_product(S.h1t, S.w2t, s0, j0, z2);
+#pragma unroll
+  for (int u = 0; u < 4; u++)
+#pragma unroll
+    for (int v = 0; v < 4; v += 2) {
+      const uint32_t hv = silu2(z2[u][v], z2[u][v + 1]);
+      S.h2t[j0 + v][s0 + u] = bf_lo(hv);
+      S.h2t[j0 + v + 1][s0 + u] = bf_hi(hv);
+    }
+  __syncthreads();
+  {  // output mo of sample s, one per thread
+    const int s = tid & 63, mo = tid >> 6;
+    float a = S.b3[mo];
+#pragma unroll 16
+    for (int j = 0; j < kH; j++) a = fmaf(S.w3[mo * kH + j], S.h2t[j][s], a);
+    S.dout[s][mo] = a;
+  }
+  __syncthreads();
+  if (tid < kTB) {  // head, loss and d loss / d o of sample tid
+    const long long s = base + tid;
+    const bool valid = S.x[tid][7] != 0.f;
+    const float o[kOut] = {S.dout[tid][0], S.dout[tid][1], S.dout[tid][2], S.dout[tid][3]};
+    float dout[kOut] = {0.f, 0.f, 0.f, 0.f};
+    float loss = 0.f;
+    if (valid) {
+      const float nx = dirs[s * 3], ny = dirs[s * 3 + 1], nz = dirs[s * 3 + 2];
+      const float na = sqrtf(fmaf(o[0], o[0], fmaf(o[1], o[1], o[2] * o[2])));
+      const float inv = 1.f / fmaxf(na, 1e-20f);
+      const float mx = o[0] * inv, my = o[1] * inv, mz = o[2] * inv;
+      const float kr = o[3] > 20.f ? o[3] : log1pf(expf(o[3]));
+      const float kappa = fminf(fmaxf(kr, kKappaMin), kappa_max);
+      const float t = fmaf(mx, nx, fmaf(my, ny, mz * nz));
+      const float at = fabsf(t);
+      const float g = kappa * (expf(kappa * (at - 1.f)) + expf(-kappa * (at + 1.f))) / (-expm1f(-2.f * kappa));
+      const float den = fmaf(1.f - kEps, g, kEps);
+      loss = -logf(den);
+      const float th = tanhf(kappa * t);
+      const float dt = -(1.f - kEps) * g * kappa * th / den;
+      const float ikc = kappa < 0.1f ? kappa * (-1.f / 3.f + kappa * kappa / 45.f) : 1.f / kappa - 1.f / tanhf(kappa);
+      float dk = -(1.f - kEps) * g * (ikc + t * th) / den;
+      if (!(kr > kKappaMin && kr < kappa_max)) dk = 0.f;
+      dout[0] = scale * dt * (nx - t * mx) * inv;
+      dout[1] = scale * dt * (ny - t * my) * inv;
+      dout[2] = scale * dt * (nz - t * mz) * inv;
+      dout[3] = scale * dk * sigm_f(o[3]);
+    }
+    S.loss[tid] = loss;
+#pragma unroll
+    for (int mo = 0; mo < kOut; mo++) S.dout[tid][mo] = dout[mo];
+  }
+  __syncthreads();
+  // backward to the hidden layers
+#pragma unroll
+  for (int u = 0; u < 4; u++)
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+      float a = 0.f;
+#pragma unroll
+      for (int mo = 0; mo < kOut; mo++) a = fmaf(S.w3[mo * kH + j0 + v], S.dout[s0 + u][mo], a);
+      const float z = z2[u][v], sg = sigm_f(z), d = a * sg * fmaf(z, 1.f - sg, 1.f);
+      S.dz2[s0 + u][j0 + v] = S.dz2t[j0 + v][s0 + u] = d;
+    }
+  __syncthreads();
+  float acc[4][4] = {};
+  tile_product(S.dz2t, S.w2, s0, j0, acc);  // sum over the units of layer 2
+#pragma unroll
+  for (int u = 0; u < 4; u++)
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+      const float z = z1[u][v], sg = sigm_f(z);
+      S.dz1[s0 + u][j0 + v] = acc[u][v] * sg * fmaf(z, 1.f - sg, 1.f);
+    }
+  __syncthreads();
+  // this block's gradients, sums over its samples in order
+  float *P = partial + (size_t)blockIdx.x * (kNP + 1);
+  {  // w2[r][c] = sum_s dz2[s][r] h1[s][c]
+    float g[4][4] = {};
+    tile_product(S.dz2, S.h1, s0, j0, g);
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+#pragma unroll
+      for (int v = 0; v < 4; v++) P[oW2 + (s0 + u) * kH + j0 + v] = g[u][v];
+  }
+  for (int i = tid; i < kH * kIn; i += kTT) {  // w1[j][k]
+    const int j = i % kH, k = i / kH;
+    float a = 0.f;
+#pragma unroll 16
+    for (int q = 0; q < kTB; q++) a = fmaf(S.dz1[q][j], S.x[q][k], a);
+    P[oW1 + j * kIn + k] = a;
+  }
+  {  // w3[mo][j]
+    const int j = tid & 63, mo = tid >> 6;
+    float a = 0.f;
+#pragma unroll 16
+    for (int q = 0; q < kTB; q++) a = fmaf(S.dout[q][mo], S.h2t[j][q], a);
+    P[oW3 + mo * kH + j] = a;
+  }
+  if (tid < 2 * kH) {  // b1, b2
+    const float (*d)[kTP] = tid < kH ? S.dz1 : S.dz2;
+    const int j = tid & 63;
+    float a = 0.f;
+#pragma unroll 16
+    for (int q = 0; q < kTB; q++) a += d[q][j];
+    P[(tid < kH ? oB1 : oB2) + j] = a;
+  } else if (tid < 2 * kH + kOut) {
+    float a = 0.f;
+    for (int q = 0; q < kTB; q++) a += S.dout[q][tid - 2 * kH];
+    P[oB3 + tid - 2 * kH] = a;
+  } else if (tid == 2 * kH + 32) {
+    float a = 0.f;
+    for (int q = 0; q < kTB; q++) a += S.loss[q];
+    P[kNP] = a;
+  }
 }
 
 // Biases stay FP32 in every pass (as in inference); weights are rounded to BF16.
@@ -874,18 +910,44 @@ __device__ __forceinline__ float pass_value(int p, float v) {
   return bias ? v : bf16r(v);
 }
 
-// Adam on the FP32 master parameters, then their copy for the next forward pass (weights BF16-rounded).
-__global__ void k_adam(const double *__restrict__ grad, float *__restrict__ params, float *__restrict__ wr,
-                       float *__restrict__ m1, float *__restrict__ m2, float lr, float bc1, float bc2) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= kNP) return;
-  const float g = (float)grad[p];
-  const float a = fmaf(0.9f, m1[p], 0.1f * g), b = fmaf(0.999f, m2[p], 0.001f * g * g);
-  m1[p] = a;
-  m2[p] = b;
-  const float v = params[p] - lr * (a / bc1) / (sqrtf(b / bc2) + 1e-8f);
-  params[p] = v;
-  wr[p] = pass_value(p, v);
+// Fixed-order FP64 sum of the block partials: the gradient, and the loss sum in out[kNP] (and in *host_loss, mapped
+// host memory, if given). With ADAM, also Adam on the FP32 master parameters and their copy for the next forward pass
+// (weights BF16-rounded): one launch, as every parameter's step needs only its own gradient.
+//
+// Bound by the latency of the sums: 32 parameters per block, their partials split over 8 warps (155 blocks), where one
+// thread per parameter added all of them in a chain on 20 SMs. Batch 8192: sum and Adam 15 us in two launches before,
+// 7 us in one now.
+constexpr int kRP = 32, kRW = 8, kRT = kRP * kRW;  // parameters and warps per block
+template <bool ADAM>
+__global__ void __launch_bounds__(kRT) k_grad_reduce(const float *__restrict__ partial, int nb, double *__restrict__ out,
+                                                     double *host_loss, float *__restrict__ params,
+                                                     float *__restrict__ wr, float *__restrict__ m1,
+                                                     float *__restrict__ m2, float lr, float bc1, float bc2) {
+  __shared__ double part[kRW][kRP];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, p = blockIdx.x * kRP + lane;
+  pdl_trigger();
+  pdl_wait();
+  double s = 0.0;
+  if (p <= kNP)
+#pragma unroll 16
+    for (int b = warp; b < nb; b += kRW) s += (double)partial[(size_t)b * (kNP + 1) + p];
+  part[warp][lane] = s;
+  __syncthreads();
+  if (warp != 0 || p > kNP) return;
+#pragma unroll
+  for (int w = 1; w < kRW; w++) s += part[w][lane];
+  out[p] = s;
+  if (p == kNP) {
+    if (host_loss) *host_loss = s;
+  } else if (ADAM) {
+    const float g = (float)s;
+    const float a = fmaf(0.9f, m1[p], 0.1f * g), b = fmaf(0.999f, m2[p], 0.001f * g * g);
+    m1[p] = a;
+    m2[p] = b;
+    const float v = params[p] - lr * (a / bc1) / (sqrtf(b / bc2) + 1e-8f);
+    params[p] = v;
+    wr[p] = pass_value(p, v);
+  }
 }
 
 __global__ void k_round(const float *__restrict__ params, float *__restrict__ wr) {
@@ -1266,6 +1328,7 @@ struct mcl_trainer {
   float kappa_max = 500.f;
   float *d_params = nullptr, *d_wr = nullptr, *d_m1 = nullptr, *d_m2 = nullptr, *d_partial = nullptr;
   double *d_grad = nullptr;
+  double *h_loss = nullptr, *d_loss = nullptr;  // the loss sum of a step: mapped host memory and its device address
   long long steps = 0;
   cudaStream_t stream = nullptr;
 };
@@ -1439,6 +1502,10 @@ int mcl_trainer_create(const mcl_mlp *init, long long max_batch, float kappa_max
   if ((err = cudaMalloc(&t->d_grad, (kNP + 1) * sizeof(double))) != cudaSuccess) return bad(err, "cudaMalloc");
   if ((err = cudaMalloc(&t->d_partial, (size_t)nb * (kNP + 1) * sizeof(float))) != cudaSuccess)
     return bad(err, "cudaMalloc");
+  if ((err = cudaHostAlloc((void **)&t->h_loss, sizeof(double), cudaHostAllocMapped)) != cudaSuccess)
+    return bad(err, "cudaHostAlloc");
+  if ((err = cudaHostGetDevicePointer((void **)&t->d_loss, t->h_loss, 0)) != cudaSuccess)
+    return bad(err, "cudaHostGetDevicePointer");
   if ((err = cudaMemcpy(t->d_params, init, kNP * sizeof(float), cudaMemcpyHostToDevice)) != cudaSuccess)
     return bad(err, "cudaMemcpy");
   if ((err = cudaMemset(t->d_m1, 0, kNP * sizeof(float))) != cudaSuccess) return bad(err, "cudaMemset");
@@ -1452,22 +1519,27 @@ int mcl_trainer_create(const mcl_mlp *init, long long max_batch, float kappa_max
   return MCL_OK;
 }
 
-static int trainer_grad(mcl_trainer *t, const float *d_features, const float *d_directors, long long n) {
+// Gradient partials of a batch and their sum; with lr > 0 the Adam step too.
+static int trainer_grad(mcl_trainer *t, const float *d_features, const float *d_directors, long long n, float lr = 0.f,
+                        float bc1 = 1.f, float bc2 = 1.f) {
+  const int nb = (int)((n + kTB - 1) / kTB);
+  CKL(launch_pdl(k_mlp_grad, nb, kTT, kTrainSmem, t->stream, t->d_wr, d_features, d_directors, n, t->kappa_max,
+                 1.f / (float)n, t->d_partial));
+  CKL(launch_pdl(lr > 0.f ? k_grad_reduce<true> : k_grad_reduce<false>, (kNP + 1 + kRP - 1) / kRP, kRT, 0, t->stream,
+                 t->d_partial, nb, t->d_grad, t->d_loss, t->d_params, t->d_wr, t->d_m1, t->d_m2, lr, bc1, bc2));
+  return MCL_OK;
+}
+
+static int trainer_check(mcl_trainer *t, const float *d_features, const float *d_directors, long long n) {
   if (!t || !d_features || !d_directors || n < 1) return fail(MCL_ERR_ARG, "trainer: bad arguments");
   if (n > t->max_batch) return fail(MCL_ERR_ARG, "trainer: batch %lld exceeds max_batch %lld", n, t->max_batch);
-  const int nb = (int)((n + kTB - 1) / kTB);
-  k_mlp_grad<<<nb, kTB, kTrainSmem, t->stream>>>(t->d_wr, d_features, d_directors, n, t->kappa_max, 1.f / (float)n,
-                                                t->d_partial);
-  CKL(cudaGetLastError());
-  k_grad_reduce<<<(kNP + 1 + 255) / 256, 256, 0, t->stream>>>(t->d_partial, nb, t->d_grad);
-  CKL(cudaGetLastError());
   return MCL_OK;
 }
 
 int mcl_trainer_gradient(mcl_trainer *t, const float *d_features, const float *d_directors, long long n,
                          mcl_mlp *grad, double *loss) {
-  int rc = trainer_grad(t, d_features, d_directors, n);
-  if (rc) return rc;
+  int rc = trainer_check(t, d_features, d_directors, n);
+  if (rc || (rc = trainer_grad(t, d_features, d_directors, n))) return rc;
   std::vector<double> g(kNP + 1);
   CKL(cudaMemcpyAsync(g.data(), t->d_grad, (kNP + 1) * sizeof(double), cudaMemcpyDeviceToHost, t->stream));
   CKL(cudaStreamSynchronize(t->stream));
@@ -1482,17 +1554,14 @@ int mcl_trainer_gradient(mcl_trainer *t, const float *d_features, const float *d
 int mcl_trainer_step(mcl_trainer *t, const float *d_features, const float *d_directors, long long n, float lr,
                      double *loss) {
   if (!(lr > 0.f && lr < 1.f)) return fail(MCL_ERR_ARG, "mcl_trainer_step: learning rate must lie in (0, 1)");
-  int rc = trainer_grad(t, d_features, d_directors, n);
+  int rc = trainer_check(t, d_features, d_directors, n);
   if (rc) return rc;
+  const float k = (float)(t->steps + 1);
+  if ((rc = trainer_grad(t, d_features, d_directors, n, lr, 1.f - powf(0.9f, k), 1.f - powf(0.999f, k)))) return rc;
   t->steps++;
-  const float bc1 = 1.f - powf(0.9f, (float)t->steps), bc2 = 1.f - powf(0.999f, (float)t->steps);
-  k_adam<<<(kNP + 255) / 256, 256, 0, t->stream>>>(t->d_grad, t->d_params, t->d_wr, t->d_m1, t->d_m2, lr, bc1, bc2);
-  CKL(cudaGetLastError());
   if (loss) {
-    double l = 0.0;
-    CKL(cudaMemcpyAsync(&l, t->d_grad + kNP, sizeof(double), cudaMemcpyDeviceToHost, t->stream));
     CKL(cudaStreamSynchronize(t->stream));
-    *loss = l / (double)n;
+    *loss = *t->h_loss / (double)n;
   }
   return MCL_OK;
 }
@@ -1513,6 +1582,7 @@ int mcl_trainer_destroy(mcl_trainer *t) {
   cudaFree(t->d_m2);
   cudaFree(t->d_grad);
   cudaFree(t->d_partial);
+  cudaFreeHost(t->h_loss);
   if (t->stream) cudaStreamDestroy(t->stream);
   delete t;
   return MCL_OK;
