@@ -769,7 +769,7 @@ static int sweeps_run(mcl_engine *e, int n, int measure) {
   const bool use_fused = e->fused && !e->record_dec && !e->d_mlp;
   if (use_fused && (rc = refresh_ghosts(e))) return rc;
   if (e->geo == GEO_PT && e->pt_lists_stale && e->schedule == MCL_SCHED_CHECKER2 && (rc = build_pt_lists(e))) return rc;
-  if (use_fused && fused_resident(e)) {
+  if (use_fused && fused_resident(e, n)) {
     // one launch for up to kResidentSweeps sweeps (bounded, so that a long call leaves the device now and then)
     constexpr int kResidentSweeps = 1024;
     while (n > 0) {
@@ -903,7 +903,7 @@ int mcl_sweeps_io(mcl_engine *e, int n, const float *T, mcl_observables *out) {
   // the sweep's kernels, output kernel reading the newest record), captured again when a buffer it uses moves.
   const bool use_fused = e->fused && !e->record_dec && !e->d_mlp;
   if (T && n == 1 && use_fused && e->use_graphs && !e->profile && fused_is_pass_plan(e)) {
-    const bool resident = fused_resident(e);
+    const bool resident = fused_resident(e, 1);
     if ((rc = ensure_series(e, e->series_len + 1))) return rc;
     if ((rc = refresh_ghosts(e))) return rc;
     if (!e->graph_io || e->graph_io_series != (const void *)e->d_series || e->graph_io_stage != e->d_io) {
@@ -1150,7 +1150,7 @@ int mcl_autotune(mcl_engine *e, int trial_sweeps, mcl_tuning *out) {
   double best = 1e300, t_default = 0;
   std::pair<int, int> pick{cfg0, seg0};
   const bool asked0 = fused_release_plan(e);
-  bool resident = fused_resident(e);  // where the engine would choose the resident kernel, it is the first candidate
+  bool resident = fused_resident(e, trial_sweeps);  // where the engine would choose the resident kernel, it is the first candidate
   const bool default_resident = resident && !asked0;
   const size_t n_cand = cand.size() + (resident ? 1 : 0);
   bool pick_resident = false;

@@ -41,9 +41,9 @@ int fused_launches_per_sweep(const mcl_engine *e);
 // rotations; zeros for the observables when measure = 0); the finalisation from such sums reduced over processes.
 bool fused_is_pass_plan(const mcl_engine *e);
 // Whether sweeps go to the resident kernel (sweep_resident.cuh): no plan was asked for, no test hook is set, every
-// replica fits a cluster's shared memory and the kernel is the faster one (resident_choose); and n of them in one
-// launch, from the buffer in use.
-bool fused_resident(const mcl_engine *e);
+// replica fits a cluster's shared memory and the kernel is the faster one for a call of n sweeps (resident_choose); and
+// n of them in one launch, from the buffer in use.
+bool fused_resident(const mcl_engine *e, int n);
 int fused_resident_sweeps(mcl_engine *e, int n, bool measure);
 // Leaves the choice of the kernel to the engine again (after fused_set_plan); returns whether a plan was asked for.
 bool fused_release_plan(mcl_engine *e);

@@ -39,6 +39,7 @@ struct FusedPlan {
   bool asked = false;          // a plan was asked for (mcl_set_plan, the autotuner, MCL_FUSED_CFG)
   int res_cluster = 0;         // CTAs per replica of the resident kernel (0: it is not used)
   size_t res_smem = 0;
+  int res_calls = 1;           // sweeps a call needs for it
 };
 
 // ---- host side ----------------------------------------------------------------------------------------------
@@ -460,7 +461,8 @@ static void resident_choose(const mcl_engine *e, FusedPlan *P) {
     return;
   }
   if (P->C.kind != 1) return;
-  double best = 5.0 + 2.0 * pass_time(e, P->cfg, P->seg, sms);  // the finalisation and the gaps between three launches
+  const double pass = 5.0 + 2.0 * pass_time(e, P->cfg, P->seg, sms);  // the finalisation and the gaps between launches
+  double best = pass;
   for (int C = 1; C <= kResMaxC && C <= min_nz; C *= 2) {
     size_t smem = 0;
     for (const auto &D : e->desc)
@@ -479,17 +481,24 @@ static void resident_choose(const mcl_engine *e, FusedPlan *P) {
       cost = std::max(cost, busy.back());
       std::push_heap(busy.begin(), busy.end(), std::greater<double>());
     }
+    // Fewer clusters than the query says may run at once, so a margin per wave.
+    const double gain = pass - cost, waves = std::ceil((double)e->n_rep / fit);
+    cost = 1.1 * cost + 3.0 * waves;
     if (cost < best) {
       best = cost;
       P->res_cluster = C;
       P->res_smem = smem;
+      // A call also reads and writes the lattice, for every wave of clusters: one sweep of 53 pear slabs of
+      // 48 x 48 x 12 per call took 151 us against 97, of 24 LL 32^3 76 against 42, of LL 20^3 33 against 29, while 20
+      // sweeps per call took 362 against 566 and 132 against 297.
+      P->res_calls = (int)std::ceil((4.0 + 10.0 * waves) / std::max(gain, 0.1));
     }
   }
 }
 
-bool fused_resident(const mcl_engine *e) {
+bool fused_resident(const mcl_engine *e, int n) {
   const FusedPlan *P = e->fused;
-  return P && P->res_cluster && !P->asked && !P->skip_first_load && !e->zslab && e->d_dir[1] == nullptr;
+  return P && P->res_cluster && n >= P->res_calls && !P->asked && !P->skip_first_load && !e->zslab && e->d_dir[1] == nullptr;
 }
 
 bool fused_release_plan(mcl_engine *e) {

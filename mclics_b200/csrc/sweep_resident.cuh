@@ -128,17 +128,27 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweep_resident(ModelDev m, R
 
   // the owned planes and their neighbours, ghost cells included (cells of an absent plane are read with weight 0)
   const int pairs_in_row = hps / 2, n2 = (nzl + 2) * (plane / 2);
-  for (int e = tid; e < n2; e += kResThreads) {
-    const int rowh = e / pairs_in_row, jj = e - rowh * pairs_in_row;  // [plane][component][y][parity], cell pair
-    const int lp = rowh / (6 * ny), in = rowh - lp * 6 * ny;
-    const int q = in / (2 * ny), yh = in - q * 2 * ny;
-    int z = z0 + lp - 1;
-    if (perz) z = z < 0 ? z + nz : (z >= nz ? z - nz : z);
-    float2 v = make_float2(0.f, 0.f);
-    if (z >= 0 && z < nz)
-      v = *reinterpret_cast<const float2 *>(gdir + q * R.comp + z * gplane + (long long)((yh >> 1) + GY) * R.px +
-                                            (yh & 1) * R.hp + GH - 2 + 2 * jj);
-    reinterpret_cast<float2 *>(planes)[e] = v;
+  constexpr int kBatch = 8;  // loads in flight per thread: one at a time, the 15-40 rounds took 10-25 us of every call
+  for (int e0 = tid; e0 < n2; e0 += kBatch * kResThreads) {
+    float2 v[kBatch];
+#pragma unroll
+    for (int i = 0; i < kBatch; i++) {
+      const int e = e0 + i * kResThreads;
+      v[i] = make_float2(0.f, 0.f);
+      if (e < n2) {
+        const int rowh = e / pairs_in_row, jj = e - rowh * pairs_in_row;  // [plane][component][y][parity], cell pair
+        const int lp = rowh / (6 * ny), in = rowh - lp * 6 * ny;
+        const int q = in / (2 * ny), yh = in - q * 2 * ny;
+        int z = z0 + lp - 1;
+        if (perz) z = z < 0 ? z + nz : (z >= nz ? z - nz : z);
+        if (z >= 0 && z < nz)
+          v[i] = *reinterpret_cast<const float2 *>(gdir + q * R.comp + z * gplane + (long long)((yh >> 1) + GY) * R.px +
+                                                   (yh & 1) * R.hp + GH - 2 + 2 * jj);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kBatch; i++)
+      if (e0 + i * kResThreads < n2) reinterpret_cast<float2 *>(planes)[e0 + i * kResThreads] = v[i];
   }
   cluster_sync();
 
