@@ -594,10 +594,11 @@ int mcl_set_geometry(mcl_engine *e, int replica, const int *pt, const float *nor
     if (pt[q] < 0 || pt[q] > 1 + e->model.n_surf)
       return fail(MCL_ERR_ARG, "point type %d at site %lld: valid are 0, 1 and 2..%d", pt[q], q, 1 + e->model.n_surf);
     p8[q] = (uint8_t)pt[q];
-    e->host_pt[D.site_off + q] = pt[q];
     nv += pt[q] != 0;
   }
   if (nv == 0) return fail(MCL_ERR_ARG, "mcl_set_geometry: no non-empty site");
+  // only now: a refused call leaves the host's point types, which the site lists and the upload's checks read, alone
+  std::copy(pt, pt + N, e->host_pt.begin() + D.site_off);
   CK(cudaMemcpyAsync(e->d_pt + D.site_off, p8.data(), N, cudaMemcpyHostToDevice, e->stream));
   CK(cudaMemcpyAsync(e->d_nrm + 3 * D.site_off, normals, N * 3 * sizeof(float), cudaMemcpyHostToDevice, e->stream));
   e->desc[replica].n_valid = (double)nv;
