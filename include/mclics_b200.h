@@ -113,6 +113,9 @@ int mcl_set_geometry(mcl_engine *e, int replica, const int *pt, const float *nor
  * zero-length directors on non-empty sites with MCL_ERR_NONFINITE and leaves the device state unchanged. */
 int mcl_upload_directors(mcl_engine *e, int replica, const float *ni);
 int mcl_download_directors(mcl_engine *e, int replica, float *ni);
+/* Downloads of 16 MiB and more (directors, local order) pass through pinned memory that the library keeps for the next
+ * one, of any engine: at most 8 MiB per process. mcl_trim gives back what no download is using. */
+int mcl_trim(void);
 
 /* Random initial condition of one replica on the device (replaces the host loop of `ic random`,
  * src/ic.cpp:38-65): every non-empty site gets an isotropic unit vector from Philox stream 2 keyed by `seed`

@@ -76,6 +76,7 @@ def lib():
         sig = {
             "mcl_create": [P(CModel), P(CReplica), i, i, P(vp)],
             "mcl_destroy": [vp],
+            "mcl_trim": [],
             "mcl_set_geometry": [vp, i, vp, vp],
             "mcl_upload_directors": [vp, i, vp],
             "mcl_download_directors": [vp, i, vp],
@@ -486,6 +487,11 @@ class Trainer:
             self.close()
         except Exception:
             pass
+
+
+def trim():
+    """Gives back the pinned memory kept between large downloads (at most 8 MiB per process)."""
+    check(lib().mcl_trim())
 
 
 def run_input_file(path):

@@ -14,6 +14,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <mutex>
 #include <thread>
 
 #include "fused.h"
@@ -77,57 +78,135 @@ static void sphere_geometry(int nx, int ny, int nz, int *pt, float *ns) {
 
 // A plain copy to pageable memory goes through the driver's staging in one thread, which also takes the page faults of a
 // fresh array: 5 GB/s, 41 ms for the 201 MB of a 256^3 field and 10.6 ms for the 50 MB of a 256 x 256 x 64 slab, most of
-// a snapshot. Here up to kCopyThreads threads each own a slot of a pinned ring: a thread queues the copy of its next
-// chunk into its slot, waits for it and moves it on, so page faults and memory copies of the chunks run side by side
-// (12 and 2.8 ms). Below kCopyLarge, where the C library hands out memory that is already mapped, a plain copy is as
-// fast (0.76 against 0.92 ms for 12.6 MB), and the ring (4 MB, 2-3 ms to pin) is not made.
-constexpr int kCopyThreads = 8;
-constexpr size_t kCopyChunk = 512 << 10, kCopyLarge = 16 << 20;
+// a snapshot. Large copies pass through a ring of pinned slots instead, one for each of up to eight threads: a thread
+// queues the copy of its next chunk into its slot, waits for it and moves it on, so page faults and memory copies of the
+// chunks run side by side (12 and 2.8 ms). The copies go to a stream of the engine's that waits for the caller's: the
+// caller's handle may name another stream in each thread (cudaStreamPerThread). Below kCopyLarge, where the C library
+// hands out memory that is already mapped, a plain copy is as fast (0.76 against 0.92 ms for 12.6 MB).
+//
+// Pinning a ring takes 3-4 ms, so rings belong to the process, at most kRings of them, and any engine takes a free one
+// (none free: a plain copy). First download of a new engine, in ms (plain copy; a ring of its own; a ring that is there):
+// 25 MB 2.5, 7.0, 1.5; 50 MB 10.4, 9.7, 4.3; 201 MB 41, 20, 13.5. The first large copy of all makes a ring only from
+// kRingWorthPinning on: below it the pinning costs what a plain copy does (25 MB into a fresh array: 7 and 5-8 ms).
+constexpr int kRings = 2;
+constexpr size_t kCopyChunk = 512 << 10, kCopyLarge = 16 << 20, kRingWorthPinning = 32 << 20;
+
+namespace {
+struct RingPool {
+  std::mutex mu;
+  char *ring[kRings] = {};
+  bool busy[kRings] = {};
+  long long asked = 0;  // large copies so far
+} g_rings;
+
+// A ring for the time of one copy of `bytes`: slots() is null when there is none to be had.
+class RingLease {
+ public:
+  explicit RingLease(size_t bytes) {
+    std::lock_guard<std::mutex> lock(g_rings.mu);
+    const bool pin = g_rings.asked++ > 0 || bytes >= kRingWorthPinning;
+    for (int i = 0; i < kRings && id_ < 0; i++)
+      if (!g_rings.busy[i] && alive(i)) id_ = i;
+    for (int i = 0; i < kRings && id_ < 0 && pin; i++)
+      if (!g_rings.busy[i]) {
+        if (cudaHostAlloc((void **)&g_rings.ring[i], kCopySlots * kCopyChunk, cudaHostAllocPortable) == cudaSuccess)
+          id_ = i;
+        else {
+          cudaGetLastError();
+          g_rings.ring[i] = nullptr;
+        }
+        break;
+      }
+    if (id_ >= 0) g_rings.busy[id_] = true;
+  }
+  ~RingLease() {
+    if (id_ < 0) return;
+    std::lock_guard<std::mutex> lock(g_rings.mu);
+    g_rings.busy[id_] = false;
+  }
+  RingLease(const RingLease &) = delete;
+  char *slots() const { return id_ < 0 ? nullptr : g_rings.ring[id_]; }
+  // Whether ring i is there and still pinned: a device reset takes pinned memory with it.
+  static bool alive(int i) {
+    if (!g_rings.ring[i]) return false;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, g_rings.ring[i]) == cudaSuccess && at.type == cudaMemoryTypeHost) return true;
+    cudaGetLastError();
+    g_rings.ring[i] = nullptr;
+    return false;
+  }
+
+ private:
+  int id_ = -1;
+};
+}  // namespace
+
+static int copy_plain(mcl_engine *e, void *dst, const void *d_src, size_t bytes) {
+  CK(cudaMemcpyAsync(dst, d_src, bytes, cudaMemcpyDeviceToHost, e->stream));
+  CK(cudaStreamSynchronize(e->stream));
+  return MCL_OK;
+}
+
+// The driver's cuCtxGetCurrent and cuCtxSetCurrent, null where they cannot be had.
+struct ContextCalls {
+  CUresult (*get)(CUcontext *) = nullptr;
+  CUresult (*set)(CUcontext) = nullptr;
+  ContextCalls() {
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", (void **)&get, cudaEnableDefault, &q) != cudaSuccess ||
+        cudaGetDriverEntryPoint("cuCtxSetCurrent", (void **)&set, cudaEnableDefault, &q) != cudaSuccess || !get || !set) {
+      cudaGetLastError();
+      get = nullptr;
+    }
+  }
+};
 
 int copy_out(mcl_engine *e, void *dst, const void *d_src, size_t bytes) {
-  const int threads = std::min<int>(kCopyThreads, std::max(1u, std::thread::hardware_concurrency() / 2));
-  if (bytes >= kCopyLarge && threads > 1) {
-    if (!e->h_copy && cudaHostAlloc((void **)&e->h_copy, kCopyThreads * kCopyChunk, cudaHostAllocDefault) != cudaSuccess) {
-      cudaGetLastError();
-      e->h_copy = nullptr;
-    }
-    while (e->h_copy && (int)e->copy_ev.size() < threads) {
-      cudaEvent_t ev;
-      CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-      e->copy_ev.push_back(ev);
-    }
-  }
-  if (bytes < kCopyLarge || threads <= 1 || !e->h_copy) {
-    CK(cudaMemcpyAsync(dst, d_src, bytes, cudaMemcpyDeviceToHost, e->stream));
-    CK(cudaStreamSynchronize(e->stream));
-    return MCL_OK;
-  }
+  static const ContextCalls context_calls;
+  const int threads = std::min<int>(kCopySlots, std::thread::hardware_concurrency() / 2);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  CUcontext ctx = nullptr;
+  if (bytes < kCopyLarge || threads < 2 || cudaStreamIsCapturing(e->stream, &capture) != cudaSuccess ||
+      capture != cudaStreamCaptureStatusNone || !context_calls.get || context_calls.get(&ctx) != CUDA_SUCCESS)
+    return copy_plain(e, dst, d_src, bytes);
+  RingLease lease(bytes);
+  char *const slots = lease.slots();
+  if (!slots) return copy_plain(e, dst, d_src, bytes);
+  if (!e->copy_stream) CK(cudaStreamCreateWithFlags(&e->copy_stream, cudaStreamNonBlocking));
+  for (cudaEvent_t &ev : e->copy_ev)
+    if (!ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  CK(cudaEventRecord(e->copy_ev[0], e->stream));
+  CK(cudaStreamWaitEvent(e->copy_stream, e->copy_ev[0], 0));
   std::atomic<int> error{(int)cudaSuccess};
   std::atomic<size_t> next{0};
   const size_t chunks = (bytes + kCopyChunk - 1) / kCopyChunk;
   auto work = [&](int t) {
-    cudaError_t err = cudaSetDevice(e->device);
-    char *slot = e->h_copy + (size_t)t * kCopyChunk;
+    cudaError_t err = cudaSuccess;
+    char *slot = slots + (size_t)t * kCopyChunk;
     for (size_t c; err == cudaSuccess && error == (int)cudaSuccess && (c = next++) < chunks;) {
       const size_t at = c * kCopyChunk, n = std::min(kCopyChunk, bytes - at);
-      err = cudaMemcpyAsync(slot, (const char *)d_src + at, n, cudaMemcpyDeviceToHost, e->stream);
-      if (err == cudaSuccess) err = cudaEventRecord(e->copy_ev[t], e->stream);
+      err = cudaMemcpyAsync(slot, (const char *)d_src + at, n, cudaMemcpyDeviceToHost, e->copy_stream);
+      if (err == cudaSuccess) err = cudaEventRecord(e->copy_ev[t], e->copy_stream);
       if (err == cudaSuccess) err = cudaEventSynchronize(e->copy_ev[t]);
       if (err == cudaSuccess) memcpy((char *)dst + at, slot, n);
     }
     if (err != cudaSuccess) error = (int)err;
   };
+  auto help = [&](int t) {
+    if (context_calls.set(ctx) == CUDA_SUCCESS) work(t);
+  };
   std::vector<std::thread> helpers;
   try {
     helpers.reserve(threads);
-    for (int t = 1; t < threads; t++) helpers.emplace_back(work, t);
+    for (int t = 1; t < threads; t++) helpers.emplace_back(help, t);
   } catch (...) {  // no more threads to be had: those there are take all chunks
   }
   work(0);
   for (std::thread &h : helpers) h.join();
-  const cudaError_t sync = cudaStreamSynchronize(e->stream);  // every slot is free again
+  const cudaError_t sync = cudaStreamSynchronize(e->copy_stream);  // every slot is free again
   if (error != (int)cudaSuccess) return cuda_fail((cudaError_t)error.load(), "device-to-host copy");
   CK(sync);
+  CK(cudaStreamSynchronize(e->stream));
   return MCL_OK;
 }
 
@@ -566,8 +645,9 @@ int mcl_destroy(mcl_engine *e) {
   cudaFree(e->d_partials);
   cudaFree(e->d_dec);
   cudaFreeHost(e->h_io);
-  cudaFreeHost(e->h_copy);
-  for (cudaEvent_t ev : e->copy_ev) cudaEventDestroy(ev);
+  for (cudaEvent_t ev : e->copy_ev)
+    if (ev) cudaEventDestroy(ev);
+  if (e->copy_stream) cudaStreamDestroy(e->copy_stream);
   for (cudaEvent_t ev : e->ev_pool) cudaEventDestroy(ev);
   if (e->own_stream) cudaStreamDestroy(e->own_stream);
   delete e;
@@ -959,6 +1039,17 @@ int mcl_sweeps_io(mcl_engine *e, int n, const float *T, mcl_observables *out) {
   if ((rc = fused_report_error(e, words[0]))) return rc;
   if ((rc = learned_report_error(e, words[1]))) return rc;
   for (size_t i = 0; i < (size_t)n * e->n_rep; i++) to_public(rec[i], out + i);
+  return MCL_OK;
+}
+
+int mcl_trim(void) {
+  std::lock_guard<std::mutex> lock(g_rings.mu);
+  for (int i = 0; i < kRings; i++)
+    if (!g_rings.busy[i] && RingLease::alive(i)) {
+      cudaFreeHost(g_rings.ring[i]);
+      g_rings.ring[i] = nullptr;
+    }
+  g_rings.asked = 0;
   return MCL_OK;
 }
 

@@ -16,7 +16,9 @@ namespace mcl {
 // Sets the thread's last error message and returns code.
 int fail(int code, const char *fmt, ...);
 int cuda_fail(cudaError_t err, const char *what);
-// Device memory to a caller's pageable memory on the engine's stream; returns when it has arrived.
+// Device memory to a caller's pageable memory on the engine's stream; returns when it has arrived. Large copies go
+// through a ring of kCopySlots pinned chunks.
+constexpr int kCopySlots = 8;
 int copy_out(mcl_engine *e, void *dst, const void *d_src, size_t bytes);
 
 struct FusedPlan;  // fused tiled sweep (sweep_fused.cu)
@@ -93,8 +95,8 @@ struct mcl_engine {
   const void *graph_series = nullptr;             // series buffer the measuring graph writes
   cudaGraphExec_t graph_io = nullptr;  // mcl_sweeps_io's step (input kernel, one measured sweep, output kernel)
   const void *graph_io_series = nullptr, *graph_io_stage = nullptr;  // the buffers it was captured with
-  char *h_copy = nullptr;    // pinned ring of large device-to-host copies (copy_out), one slot per copying thread
-  std::vector<cudaEvent_t> copy_ev;
+  cudaStream_t copy_stream = nullptr;  // of large device-to-host copies (copy_out)
+  cudaEvent_t copy_ev[mcl::kCopySlots] = {};  // one per slot of a ring
   void *h_io = nullptr;      // mapped pinned staging of mcl_sweeps_io: error words, temperatures, observables records
   void *d_io = nullptr;      // its device address
   size_t h_io_bytes = 0;
