@@ -210,7 +210,7 @@ int copy_out(mcl_engine *e, void *dst, const void *d_src, size_t bytes) {
   return MCL_OK;
 }
 
-static int build_table(BlockTable &t, const std::vector<long long> &items, int threads) {
+static int build_table(BlockTable &t, const std::vector<long long> &items, int threads, cudaStream_t stream) {
   std::vector<int> rep, first;
   std::vector<long long> base;
   for (size_t r = 0; r < items.size(); r++) {
@@ -223,12 +223,12 @@ static int build_table(BlockTable &t, const std::vector<long long> &items, int t
   first.push_back((int)rep.size());
   t.n_blocks = (int)rep.size();
   CK(cudaMalloc(&t.first, first.size() * sizeof(int)));
-  CK(cudaMemcpy(t.first, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice));
+  CK(copy_in(stream, t.first, first.data(), first.size() * sizeof(int)));
   if (t.n_blocks) {
     CK(cudaMalloc(&t.rep, rep.size() * sizeof(int)));
     CK(cudaMalloc(&t.base, base.size() * sizeof(long long)));
-    CK(cudaMemcpy(t.rep, rep.data(), rep.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(t.base, base.data(), base.size() * sizeof(long long), cudaMemcpyHostToDevice));
+    CK(copy_in(stream, t.rep, rep.data(), rep.size() * sizeof(int)));
+    CK(copy_in(stream, t.base, base.data(), base.size() * sizeof(long long)));
   }
   return MCL_OK;
 }
@@ -307,9 +307,9 @@ static int build_pt_lists(mcl_engine *e) {
     free_pt_lists(t);
     return MCL_OK;
   }
-  CK(cudaMemcpy(t.sites, sites.data(), sites.size() * sizeof(PtSite), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(t.blocks, blocks.data(), blocks.size() * sizeof(PtBlock), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(t.first, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice));
+  CK(copy_in(e->stream, t.sites, sites.data(), sites.size() * sizeof(PtSite)));
+  CK(copy_in(e->stream, t.blocks, blocks.data(), blocks.size() * sizeof(PtBlock)));
+  CK(copy_in(e->stream, t.first, first.data(), first.size() * sizeof(int)));
   t.n_blocks = (int)blocks.size();
   return MCL_OK;
 }
@@ -568,8 +568,8 @@ int mcl_create(const mcl_model *model, const mcl_replica *replicas, int n_replic
         e->geometry_set = false;  // custom: mcl_set_geometry required before sweeping
     }
     std::vector<uint8_t> p8(e->host_pt.begin(), e->host_pt.end());
-    CKC(cudaMemcpy(e->d_pt, p8.data(), p8.size(), cudaMemcpyHostToDevice));
-    CKC(cudaMemcpy(e->d_nrm, ns.data(), ns.size() * sizeof(float), cudaMemcpyHostToDevice));
+    CKC(copy_in(e->stream, e->d_pt, p8.data(), p8.size()));
+    CKC(copy_in(e->stream, e->d_nrm, ns.data(), ns.size() * sizeof(float)));
     for (int r = 0; r < n_replicas; r++) {
       const RepDesc &D = e->desc[r];
       long long nv = 0;
@@ -577,8 +577,8 @@ int mcl_create(const mcl_model *model, const mcl_replica *replicas, int n_replic
       e->desc[r].n_valid = (double)nv;
     }
   }
-  CKC(cudaMemcpy(e->d_desc, e->desc.data(), n_replicas * sizeof(RepDesc), cudaMemcpyHostToDevice));
-  CKC(cudaMemcpy(e->d_state, st.data(), n_replicas * sizeof(RepState), cudaMemcpyHostToDevice));
+  CKC(copy_in(e->stream, e->d_desc, e->desc.data(), n_replicas * sizeof(RepDesc)));
+  CKC(copy_in(e->stream, e->d_state, st.data(), n_replicas * sizeof(RepState)));
 
   std::vector<long long> half, boxes, sites;
   for (auto &D : e->desc) {
@@ -587,9 +587,9 @@ int mcl_create(const mcl_model *model, const mcl_replica *replicas, int n_replic
     sites.push_back((long long)D.nx * D.ny * D.nz);
   }
   int rc;
-  if ((rc = build_table(e->half, half, kThreads)) != MCL_OK) return cleanup_fail(rc);
-  if ((rc = build_table(e->boxes, boxes, kThreads)) != MCL_OK) return cleanup_fail(rc);
-  if ((rc = build_table(e->sites, sites, kThreads)) != MCL_OK) return cleanup_fail(rc);
+  if ((rc = build_table(e->half, half, kThreads, e->stream)) != MCL_OK) return cleanup_fail(rc);
+  if ((rc = build_table(e->boxes, boxes, kThreads, e->stream)) != MCL_OK) return cleanup_fail(rc);
+  if ((rc = build_table(e->sites, sites, kThreads, e->stream)) != MCL_OK) return cleanup_fail(rc);
   CKC(cudaMalloc(&e->d_partials, (size_t)std::max(1, e->sites.n_blocks) * kPartials * sizeof(double)));
 
   // directors start at (0, 0, 1) (the reference's value for unset sites)
@@ -600,7 +600,7 @@ int mcl_create(const mcl_model *model, const mcl_replica *replicas, int n_replic
       aos[3 * q + 1] = 0.f;
       aos[3 * q + 2] = 1.f;
     }
-    CKC(cudaMemcpy(e->d_stage, aos.data(), aos.size() * sizeof(float), cudaMemcpyHostToDevice));
+    CKC(copy_in(e->stream, e->d_stage, aos.data(), aos.size() * sizeof(float)));
     for (int r = 0; r < n_replicas; r++) CKC(launch_unpack(e->ctx(), r, e->desc[r], e->d_stage));
   }
   if (schedule == MCL_SCHED_CHECKER2 && fused_supported(e)) {
@@ -1333,7 +1333,7 @@ int mcl_zslab_init(mcl_engine *e, int nz_global, int z_offset, int periodic_z, l
   D.nzg = nz_global;
   D.periodic[2] = periodic_z ? 1 : 0;
   D.n_valid = (double)D.nx * D.ny * nz_global;
-  CK(cudaMemcpy(e->d_desc, &D, sizeof D, cudaMemcpyHostToDevice));
+  CK(copy_in(e->stream, e->d_desc, &D, sizeof D));
   e->zslab = true;
   drop_graphs(e);
   const bool flip = e->model.flip != 0 || e->model.potential == POT_PEAR;

@@ -16,6 +16,12 @@ namespace mcl {
 // Sets the thread's last error message and returns code.
 int fail(int code, const char *fmt, ...);
 int cuda_fail(cudaError_t err, const char *what);
+// Host memory that a set-up prepared, to the device, complete on return. On the stream whose kernels read it: the
+// library's streams do not wait for the default stream, whose copies from pageable memory may return before they end.
+inline cudaError_t copy_in(cudaStream_t stream, void *d_dst, const void *src, size_t bytes) {
+  const cudaError_t err = cudaMemcpyAsync(d_dst, src, bytes, cudaMemcpyHostToDevice, stream);
+  return err != cudaSuccess ? err : cudaStreamSynchronize(stream);
+}
 // Device memory to a caller's pageable memory on the engine's stream; returns when it has arrived. Large copies go
 // through a ring of kCopySlots pinned chunks.
 constexpr int kCopySlots = 8;

@@ -1379,10 +1379,10 @@ int mcl_set_proposal(mcl_engine *e, const mcl_mlp *mlp, float kappa_max) {
   if (!e->d_mlp_tc) CKL(cudaMalloc(&e->d_mlp_tc, sizeof(MlpTC)));
   if (!e->d_lerr) {
     CKL(cudaMalloc(&e->d_lerr, sizeof(unsigned)));
-    CKL(cudaMemset(e->d_lerr, 0, sizeof(unsigned)));
+    CKL(cudaMemsetAsync(e->d_lerr, 0, sizeof(unsigned), e->stream));
   }
-  CKL(cudaMemcpy(e->d_mlp, &h, sizeof h, cudaMemcpyHostToDevice));
-  CKL(cudaMemcpy(e->d_mlp_tc, &ht, sizeof ht, cudaMemcpyHostToDevice));
+  CKL(copy_in(e->stream, e->d_mlp, &h, sizeof h));
+  CKL(copy_in(e->stream, e->d_mlp_tc, &ht, sizeof ht));
   e->kappa_max = kappa_max;
   // tcgen05 unless MCL_LEARNED_MLP=mma selects the mma.sync warps (same network, same rounding points)
   const char *path = getenv("MCL_LEARNED_MLP");
@@ -1506,10 +1506,9 @@ int mcl_trainer_create(const mcl_mlp *init, long long max_batch, float kappa_max
     return bad(err, "cudaHostAlloc");
   if ((err = cudaHostGetDevicePointer((void **)&t->d_loss, t->h_loss, 0)) != cudaSuccess)
     return bad(err, "cudaHostGetDevicePointer");
-  if ((err = cudaMemcpy(t->d_params, init, kNP * sizeof(float), cudaMemcpyHostToDevice)) != cudaSuccess)
-    return bad(err, "cudaMemcpy");
-  if ((err = cudaMemset(t->d_m1, 0, kNP * sizeof(float))) != cudaSuccess) return bad(err, "cudaMemset");
-  if ((err = cudaMemset(t->d_m2, 0, kNP * sizeof(float))) != cudaSuccess) return bad(err, "cudaMemset");
+  if ((err = copy_in(t->stream, t->d_params, init, kNP * sizeof(float))) != cudaSuccess) return bad(err, "copy_in");
+  if ((err = cudaMemsetAsync(t->d_m1, 0, kNP * sizeof(float), t->stream)) != cudaSuccess) return bad(err, "cudaMemset");
+  if ((err = cudaMemsetAsync(t->d_m2, 0, kNP * sizeof(float), t->stream)) != cudaSuccess) return bad(err, "cudaMemset");
   k_round<<<(kNP + 255) / 256, 256, 0, t->stream>>>(t->d_params, t->d_wr);
   if ((err = cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem)) !=
       cudaSuccess)
@@ -1568,8 +1567,8 @@ int mcl_trainer_step(mcl_trainer *t, const float *d_features, const float *d_dir
 
 int mcl_trainer_get(mcl_trainer *t, mcl_mlp *out) {
   if (!t || !out) return fail(MCL_ERR_ARG, "mcl_trainer_get: null argument");
+  CKL(cudaMemcpyAsync(out, t->d_params, kNP * sizeof(float), cudaMemcpyDeviceToHost, t->stream));
   CKL(cudaStreamSynchronize(t->stream));
-  CKL(cudaMemcpy(out, t->d_params, kNP * sizeof(float), cudaMemcpyDeviceToHost));
   return MCL_OK;
 }
 

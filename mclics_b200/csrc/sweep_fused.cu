@@ -235,7 +235,7 @@ static int build_items(mcl_engine *e, FusedPlan *P) {
   cudaFree(P->d_first);
   cudaFree(P->d_partials);
   CKF(cudaMalloc(&P->d_tmaps, maps.size() * sizeof(CUtensorMap)));
-  CKF(cudaMemcpy(P->d_tmaps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
+  CKF(copy_in(e->stream, P->d_tmaps, maps.data(), maps.size() * sizeof(CUtensorMap)));
   std::vector<FusedItem> items;
   std::vector<int> first;
   for (int r = 0; r < e->n_rep; r++) {
@@ -249,9 +249,9 @@ static int build_items(mcl_engine *e, FusedPlan *P) {
   first.push_back((int)items.size());
   P->n_items = (int)items.size();
   CKF(cudaMalloc(&P->d_items, items.size() * sizeof(FusedItem)));
-  CKF(cudaMemcpy(P->d_items, items.data(), items.size() * sizeof(FusedItem), cudaMemcpyHostToDevice));
+  CKF(copy_in(e->stream, P->d_items, items.data(), items.size() * sizeof(FusedItem)));
   CKF(cudaMalloc(&P->d_first, first.size() * sizeof(int)));
-  CKF(cudaMemcpy(P->d_first, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice));
+  CKF(copy_in(e->stream, P->d_first, first.data(), first.size() * sizeof(int)));
   CKF(cudaMalloc(&P->d_partials, (size_t)P->n_items * kPartials * sizeof(double)));
   const bool pass = P->C.kind == 1;
   const int nsl = pass ? NSLP : NSL;
@@ -266,7 +266,7 @@ int fused_create(mcl_engine *e) {
   P->cfg = choose_cfg(e);
   P->asked = getenv("MCL_FUSED_CFG") != nullptr;
   CKF(cudaMalloc(&P->d_err, sizeof(unsigned int)));
-  CKF(cudaMemset(P->d_err, 0, sizeof(unsigned int)));
+  CKF(cudaMemsetAsync(P->d_err, 0, sizeof(unsigned int), e->stream));
   const int rc = build_items(e, P);
   if (rc == MCL_OK) resident_choose(e, P);
   return rc;
@@ -663,8 +663,7 @@ unsigned int *fused_error_word(mcl_engine *e) { return e->fused ? e->fused->d_er
 
 int fused_report_error(mcl_engine *e, unsigned int v) {
   if (!v || !e->fused) return MCL_OK;
-  unsigned int zero = 0;
-  CKF(cudaMemcpy(e->fused->d_err, &zero, sizeof zero, cudaMemcpyHostToDevice));
+  CKF(cudaMemsetAsync(e->fused->d_err, 0, sizeof v, e->stream));
   return fail(MCL_ERR_CUDA, "fused sweep: a TMA load did not complete within %.3f s (error word 0x%x)",
               e->fused->timeout_ns * 1e-9, v);
 }
