@@ -34,6 +34,7 @@ int fail(int code, const char *fmt, ...) {
 }
 
 int cuda_fail(cudaError_t err, const char *what) {
+  cudaGetLastError();  // reported here: the next launch's check must not find it again
   return fail(err == cudaErrorMemoryAllocation ? MCL_ERR_NOMEM : MCL_ERR_CUDA, "%s: %s (%s)", what,
               cudaGetErrorString(err), cudaGetErrorName(err));
 }
