@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <atomic>
 #include <mutex>
+#include <new>
 #include <thread>
 
 #include "fused.h"
@@ -248,15 +249,9 @@ static void free_pt_lists(PtLists &t) {
   t = PtLists();
 }
 
-// The site lists of the point-type sweep from the engine's point types. If the device has no room for them, the engine
-// goes on with the kernel that needs none (no list: n_blocks = 0).
-static int build_pt_lists(mcl_engine *e) {
-  CK(cudaStreamSynchronize(e->stream));
-  free_pt_lists(e->pt_lists);
-  e->pt_lists_stale = false;
-  std::vector<PtSite> sites;
-  std::vector<PtBlock> blocks;
-  std::vector<int> first;
+// The non-empty sites of every replica, colour by colour, and the blocks that sweep them (PtLists).
+static void list_sites(const mcl_engine *e, std::vector<PtSite> &sites, std::vector<PtBlock> &blocks,
+                       std::vector<int> &first) {
   std::vector<PtSite> other;  // colour 1 of the replica at hand
   for (int r = 0; r < e->n_rep; r++) {
     const RepDesc &D = e->desc[r];
@@ -298,6 +293,22 @@ static int build_pt_lists(mcl_engine *e) {
     }
   }
   first.push_back((int)blocks.size());
+}
+
+// The site lists of the point-type sweep from the engine's point types. If the host or the device has no room for
+// them, the engine goes on with the kernel that needs none (no list: n_blocks = 0).
+static int build_pt_lists(mcl_engine *e) {
+  CK(cudaStreamSynchronize(e->stream));
+  free_pt_lists(e->pt_lists);
+  e->pt_lists_stale = false;
+  std::vector<PtSite> sites;
+  std::vector<PtBlock> blocks;
+  std::vector<int> first;
+  try {
+    list_sites(e, sites, blocks, first);
+  } catch (const std::bad_alloc &) {
+    return MCL_OK;
+  }
   // one row of partials per block, in the engine's buffer (a block per 256 sites of the box)
   if (blocks.empty() || (long long)blocks.size() > (long long)e->sites.n_blocks) return MCL_OK;
   PtLists &t = e->pt_lists;
