@@ -861,7 +861,16 @@ static int sweeps_run(mcl_engine *e, int n, int measure) {
   if (measure && (rc = ensure_series(e, e->series_len + n))) return rc;
   const bool use_fused = e->fused && !e->record_dec && !e->d_mlp;
   if (use_fused && (rc = refresh_ghosts(e))) return rc;
-  if (e->geo == GEO_PT && e->pt_lists_stale && e->schedule == MCL_SCHED_CHECKER2 && (rc = build_pt_lists(e))) return rc;
+  // Point types by site lists, except in a capture of the caller's: building them waits for the device, and the graph
+  // would keep the lists of a geometry that may have been replaced when it is replayed.
+  bool by_lists = e->geo == GEO_PT && e->schedule == MCL_SCHED_CHECKER2 && !e->record_dec;
+  if (by_lists) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(e->stream, &capture));
+    by_lists = capture == cudaStreamCaptureStatusNone;
+    if (by_lists && e->pt_lists_stale && (rc = build_pt_lists(e))) return rc;
+    by_lists = by_lists && e->pt_lists.n_blocks > 0;
+  }
   if (use_fused && fused_resident(e, n)) {
     // one launch for up to kResidentSweeps sweeps (bounded, so that a long call leaves the device now and then)
     constexpr int kResidentSweeps = 1024;
@@ -928,7 +937,7 @@ static int sweeps_run(mcl_engine *e, int n, int measure) {
         if (measure) e->series_len++;
         continue;
       }
-      if (e->pt_lists.n_blocks && e->schedule == MCL_SCHED_CHECKER2 && !e->record_dec) {  // point types, by site lists
+      if (by_lists) {
         CK(launch_sweep_pt(c, e->pt_lists, measure ? 1 : 0, e->d_partials));
         e->launches += 2;
         if (ev1) CK(cudaEventRecord(ev1, e->stream));
