@@ -795,13 +795,19 @@ static int sweeps_run(mcl_engine *e, int n, int measure);
 
 static int sweeps_all(mcl_engine *e, int n, int measure);
 
+// S and director of the series records from row `first` on.
+static cudaError_t solve_records(mcl_engine *e, int first) {
+  if (e->series_len == first) return cudaSuccess;
+  e->launches++;
+  return launch_series_eigen(e->stream, e->d_series, (long long)first * e->n_rep,
+                             (long long)(e->series_len - first) * e->n_rep);
+}
+
 int mcl_sweeps(mcl_engine *e, int n, int measure) {
   const int first = e ? e->series_len : 0;
   const int rc = sweeps_all(e, n, measure);
-  if (!e || !measure || e->series_len == first) return rc;
-  const long long rows = e->series_len - first;  // also after an error: the sweeps that were queued have records
-  const cudaError_t ce = launch_series_eigen(e->stream, e->d_series, (long long)first * e->n_rep, rows * e->n_rep);
-  e->launches++;
+  if (!e || !measure) return rc;
+  const cudaError_t ce = solve_records(e, first);  // also after an error: the sweeps that were queued have records
   if (rc) return rc;
   CK(ce);
   return MCL_OK;
@@ -1049,7 +1055,10 @@ int mcl_sweeps_io(mcl_engine *e, int n, const float *T, mcl_observables *out) {
       e->launches++;
     }
     const int first = e->series_len;
-    if ((rc = sweeps_all(e, n, 1))) return rc;
+    if ((rc = sweeps_all(e, n, 1))) {
+      solve_records(e, first);
+      return rc;
+    }
     e->io_inflight = true;
     CK(launch_io_out(e->stream, e->d_series, first, nullptr, n, e->n_rep, (ObsRecord *)(dio + rec_off),
                      fused_error_word(e), e->d_lerr, (unsigned *)dio));
