@@ -216,14 +216,16 @@ int mcl_local_order(mcl_engine *e, int replica, float *S);
  *   4: colour passes, 32 x 16 sites, 128 threads, 5 CTAs per SM (narrow lattices waste less of a tile).
  * Without a plan asked for (mcl_set_plan, mcl_autotune), an engine whose replicas are small sweeps them in shared
  * memory instead, one cluster of CTAs per replica and all sweeps of a call in one launch; mcl_get_plan then names the
- * tile plan it would use otherwise. mcl_autotune times that kernel too and, where it is the fastest, keeps it (the
- * plan fields of *out are then the default plan's).
+ * tile plan it would use otherwise. mcl_autotune times that kernel too, over calls long enough for it, and leaves the
+ * choice to the engine where it is the fastest; the plan fields of *out are then those of the fastest colour-pass plan,
+ * which shorter calls run.
  * The fused configurations need a second director buffer, allocated while one of them is selected and freed when a
  * colour-pass configuration is selected again. Every configuration gives bit-identical directors. Candidate plans:
  * per configuration the heuristic segment length, its double, its half and the whole depth; lattices that give
  * fewer work items than SMs also 2-4 planes in the colour passes. mcl_autotune times each candidate plan for
  * trial_sweeps measured sweeps on the engine's own replicas, keeps the fastest and restores the directors,
- * per-replica state, sweep counter and series, so the run continues as if it had not been called. MCL_ERR_STATE
+ * per-replica state, sweep counter and series, so the run continues as if it had not been called; if it fails, the
+ * plan stays what it was too. MCL_ERR_STATE
  * unless the engine runs the tiled sweep (bulk/slab, plain proposal, no decision recording). */
 typedef struct mcl_tuning {
   int tile_config;        /* 0..4 as above */

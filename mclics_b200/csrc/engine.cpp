@@ -1218,7 +1218,11 @@ int mcl_autotune(mcl_engine *e, int trial_sweeps, mcl_tuning *out) {
   if (!e->fused || e->record_dec || e->d_mlp || e->zslab)
     return fail(MCL_ERR_STATE, "mcl_autotune: the engine does not run the tiled sweep of whole lattices");
   int rc;
-  if ((rc = ensure_series(e, e->series_len + trial_sweeps + 1))) return rc;
+  // where the resident kernel can run it is a candidate, timed over calls long enough for it: at four times the length
+  // from which it is chosen, most of what it gains on long calls shows
+  const int res_calls = fused_resident_calls(e);
+  const int res_sweeps = std::max(trial_sweeps, (int)std::min(10000ll, 4ll * res_calls));
+  if ((rc = ensure_series(e, e->series_len + res_sweeps + std::max(1, res_calls)))) return rc;
   CK(cudaStreamSynchronize(e->stream));
   // state to restore: directors (with ghosts), per-replica state, sweep counter, series length
   float *save = nullptr;
@@ -1228,7 +1232,28 @@ int mcl_autotune(mcl_engine *e, int trial_sweeps, mcl_tuning *out) {
   std::vector<RepState> st(e->n_rep);
   unsigned long long sweep0 = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  const FusedChoice plan0 = fused_choice(e);
+  bool saved = false;
+  // the candidate plan decides whether a second buffer exists: the state always goes back into buffer 0
+  auto restore = [&]() -> int {
+    e->cur = 0;
+    CK(cudaMemcpyAsync(e->d_dir[0], save, (size_t)e->dir_floats * sizeof(float), cudaMemcpyDeviceToDevice,
+                       e->stream));
+    CK(cudaMemcpyAsync(e->d_state, st.data(), e->n_rep * sizeof(RepState), cudaMemcpyHostToDevice, e->stream));
+    CK(cudaMemcpyAsync(e->d_sweep, &sweep0, sizeof sweep0, cudaMemcpyHostToDevice, e->stream));
+    CK(cudaMemcpyAsync(e->d_series_len, &series0, sizeof series0, cudaMemcpyHostToDevice, e->stream));
+    e->series_len = series0;
+    e->ghosts_dirty = false;  // the saved buffer carries its ghost cells
+    CK(cudaStreamSynchronize(e->stream));
+    return MCL_OK;
+  };
   auto done = [&](int code) {
+    if (code != MCL_OK && saved) {  // plan and state as they were, and the first error's message
+      const std::string message = g_err;
+      fused_restore(e, plan0);
+      restore();
+      g_err = message;
+    }
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     cudaFree(save);
@@ -1246,19 +1271,7 @@ int mcl_autotune(mcl_engine *e, int trial_sweeps, mcl_tuning *out) {
   CKT(cudaMemcpyAsync(st.data(), e->d_state, e->n_rep * sizeof(RepState), cudaMemcpyDeviceToHost, e->stream));
   CKT(cudaMemcpyAsync(&sweep0, e->d_sweep, sizeof sweep0, cudaMemcpyDeviceToHost, e->stream));
   CKT(cudaStreamSynchronize(e->stream));
-  // the candidate plan decides whether a second buffer exists: the state always goes back into buffer 0
-  auto restore = [&]() -> int {
-    e->cur = 0;
-    CK(cudaMemcpyAsync(e->d_dir[0], save, (size_t)e->dir_floats * sizeof(float), cudaMemcpyDeviceToDevice,
-                       e->stream));
-    CK(cudaMemcpyAsync(e->d_state, st.data(), e->n_rep * sizeof(RepState), cudaMemcpyHostToDevice, e->stream));
-    CK(cudaMemcpyAsync(e->d_sweep, &sweep0, sizeof sweep0, cudaMemcpyHostToDevice, e->stream));
-    CK(cudaMemcpyAsync(e->d_series_len, &series0, sizeof series0, cudaMemcpyHostToDevice, e->stream));
-    e->series_len = series0;
-    e->ghosts_dirty = false;  // the saved buffer carries its ghost cells
-    CK(cudaStreamSynchronize(e->stream));
-    return MCL_OK;
-  };
+  saved = true;
   drop_graphs(e);
   e->use_graphs = false;
   e->profile = false;
@@ -1269,36 +1282,50 @@ int mcl_autotune(mcl_engine *e, int trial_sweeps, mcl_tuning *out) {
   std::vector<std::pair<int, int>> cand;
   fused_plan_candidates(e, cand);
   if (std::find(cand.begin(), cand.end(), std::make_pair(cfg0, seg0)) == cand.end()) cand.push_back({cfg0, seg0});
-  double best = 1e300, t_default = 0;
-  std::pair<int, int> pick{cfg0, seg0};
-  const bool asked0 = fused_release_plan(e);
-  bool resident = fused_resident(e, trial_sweeps);  // where the engine would choose the resident kernel, it is the first candidate
-  const bool default_resident = resident && !asked0;
-  const size_t n_cand = cand.size() + (resident ? 1 : 0);
-  bool pick_resident = false;
-  if (resident) cand.insert(cand.begin(), {cfg0, seg0});
-  for (const auto &c : cand) {
-    if (!resident && (rc = fused_set_plan(e, c.first, c.second))) return done(rc);
-    if ((rc = mcl_sweeps(e, 1, 1))) return done(rc);  // warm-up
-    CKT(cudaEventRecord(ev0, e->stream));
-    if ((rc = mcl_sweeps(e, trial_sweeps, 1))) return done(rc);
-    CKT(cudaEventRecord(ev1, e->stream));
-    CKT(cudaEventSynchronize(ev1));
+  // ms per sweep of a call of n sweeps, after a call of `warm` sweeps; then the state goes back
+  auto timed = [&](int warm, int n, double *per) -> int {
+    int rc2;
+    if ((rc2 = mcl_sweeps(e, warm, 1))) return rc2;
+    CK(cudaEventRecord(ev0, e->stream));
+    if ((rc2 = mcl_sweeps(e, n, 1))) return rc2;
+    CK(cudaEventRecord(ev1, e->stream));
+    CK(cudaEventSynchronize(ev1));
     float ms = 0.f;
-    CKT(cudaEventElapsedTime(&ms, ev0, ev1));
-    const double per = ms / trial_sweeps;
-    if (default_resident ? resident : (!resident && c.first == cfg0 && c.second == seg0)) t_default = per;
+    CK(cudaEventElapsedTime(&ms, ev0, ev1));
+    *per = ms / n;
+    if ((rc2 = restore())) return rc2;
+    return fused_check_error(e);
+  };
+  double best = 1e300, best_pass = 1e300, t_default = 0, per = 0;
+  std::pair<int, int> pick{cfg0, seg0}, pick_pass = pick;  // the fastest plan, and the fastest of the colour passes
+  const size_t n_cand = cand.size() + (res_calls ? 1 : 0);
+  double t_resident = 1e300;
+  if (res_calls) {
+    fused_release_plan(e);
+    if ((rc = timed(res_calls, res_sweeps, &t_resident))) return done(rc);
+    if (!plan0.asked) t_default = t_resident;
+  }
+  for (const auto &c : cand) {
+    if ((rc = fused_set_plan(e, c.first, c.second))) return done(rc);
+    const bool pass = fused_is_pass_plan(e);
+    if ((rc = timed(1, trial_sweeps, &per))) return done(rc);
+    if ((plan0.asked || !res_calls) && c.first == cfg0 && c.second == seg0) t_default = per;
     if (per < best) {
       best = per;
       pick = c;
-      pick_resident = resident;
     }
-    resident = false;
-    if ((rc = restore())) return done(rc);
-    if ((rc = fused_check_error(e))) return done(rc);
+    if (pass && per < best_pass) {
+      best_pass = per;
+      pick_pass = c;
+    }
+  }
+  const bool resident = t_resident < best;  // in long calls; shorter ones run the fastest colour passes
+  if (resident) {
+    best = t_resident;
+    pick = pick_pass;
   }
   if ((rc = fused_set_plan(e, pick.first, pick.second))) return done(rc);
-  if (pick_resident) fused_release_plan(e);
+  if (resident) fused_release_plan(e);
   if (out) {
     int ty = 0, seg = 0, items = 0;
     fused_get_cfg(e, nullptr, &ty, &seg, &items);

@@ -45,8 +45,17 @@ bool fused_is_pass_plan(const mcl_engine *e);
 // n of them in one launch, from the buffer in use.
 bool fused_resident(const mcl_engine *e, int n);
 int fused_resident_sweeps(mcl_engine *e, int n, bool measure);
-// Leaves the choice of the kernel to the engine again (after fused_set_plan); returns whether a plan was asked for.
-bool fused_release_plan(mcl_engine *e);
+// The sweeps a call needs for the resident kernel where no plan is asked for (0: the engine does not use it).
+int fused_resident_calls(const mcl_engine *e);
+// Leaves the choice of the kernel to the engine again (after fused_set_plan).
+void fused_release_plan(mcl_engine *e);
+// The plan with all that was asked for, and the way back to it.
+struct FusedChoice {
+  int cfg, seg_override;
+  bool asked;
+};
+FusedChoice fused_choice(const mcl_engine *e);
+int fused_restore(mcl_engine *e, const FusedChoice &c);
 // Work items, tensor maps and partials of the learned colour passes' own plan (64 x 8 tiles), built at the first
 // call; MCL_ERR_STATE without the tiled sweep.
 int fused_learned_view(mcl_engine *e, LearnedPassView *v);

@@ -496,15 +496,24 @@ static void resident_choose(const mcl_engine *e, FusedPlan *P) {
   }
 }
 
-bool fused_resident(const mcl_engine *e, int n) {
+int fused_resident_calls(const mcl_engine *e) {
   const FusedPlan *P = e->fused;
-  return P && P->res_cluster && n >= P->res_calls && !P->asked && !P->skip_first_load && !e->zslab && e->d_dir[1] == nullptr;
+  return P && P->res_cluster && !P->skip_first_load && !e->zslab && e->d_dir[1] == nullptr ? P->res_calls : 0;
 }
 
-bool fused_release_plan(mcl_engine *e) {
-  const bool asked = e->fused && e->fused->asked;
-  if (e->fused) e->fused->asked = false;
-  return asked;
+bool fused_resident(const mcl_engine *e, int n) {
+  const int calls = fused_resident_calls(e);
+  return calls > 0 && n >= calls && !e->fused->asked;
+}
+
+void fused_release_plan(mcl_engine *e) { e->fused->asked = false; }
+
+FusedChoice fused_choice(const mcl_engine *e) { return {e->fused->cfg, e->fused->seg_override, e->fused->asked}; }
+
+int fused_restore(mcl_engine *e, const FusedChoice &c) {
+  CKF(cudaStreamSynchronize(e->stream));
+  e->fused->asked = c.asked;
+  return apply_plan(e, c.cfg, c.seg_override);
 }
 
 int fused_resident_sweeps(mcl_engine *e, int n, bool measure) {
