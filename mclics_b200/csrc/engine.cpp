@@ -1228,7 +1228,7 @@ int mcl_autotune(mcl_engine *e, int trial_sweeps, mcl_tuning *out) {
   float *save = nullptr;
   CK(cudaMalloc(&save, (size_t)e->dir_floats * sizeof(float)));
   const int cur0 = e->cur, series0 = e->series_len;
-  const bool graphs0 = e->use_graphs, prof0 = e->profile;
+  const bool graphs0 = e->use_graphs, prof0 = e->profile, ghosts0 = e->ghosts_dirty;
   std::vector<RepState> st(e->n_rep);
   unsigned long long sweep0 = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -1243,7 +1243,7 @@ int mcl_autotune(mcl_engine *e, int trial_sweeps, mcl_tuning *out) {
     CK(cudaMemcpyAsync(e->d_sweep, &sweep0, sizeof sweep0, cudaMemcpyHostToDevice, e->stream));
     CK(cudaMemcpyAsync(e->d_series_len, &series0, sizeof series0, cudaMemcpyHostToDevice, e->stream));
     e->series_len = series0;
-    e->ghosts_dirty = false;  // the saved buffer carries its ghost cells
+    e->ghosts_dirty = ghosts0;  // the ghost cells are those of the saved buffer
     CK(cudaStreamSynchronize(e->stream));
     return MCL_OK;
   };
