@@ -304,7 +304,8 @@ int mcl_set_proposal_mix(mcl_engine *e, int period);
 int mcl_set_adaptation(mcl_engine *e, int enable);
 /* Training samples from the current state of one replica: n sites drawn with Philox(seed, sample index). Device
  * buffers: d_features n x 8 floats (7 features, then 1 for a non-empty site / 0 for an empty one), d_directors
- * n x 3 floats (the site's director). Synchronises. */
+ * n x 3 floats (the site's director). The engine's stream waits for no other: work queued elsewhere on the buffers
+ * must have ended. Synchronises. */
 int mcl_extract_samples(mcl_engine *e, int replica, long long n, unsigned long long seed, float *d_features,
                         float *d_directors);
 /* The tensor-core MLP on n feature rows (device, n x 8 floats as above) -> d_out n x 4 raw outputs (before the
@@ -317,7 +318,9 @@ int mcl_mlp_forward_tcgen05(const mcl_mlp *mlp, const float *d_features, long lo
 
 /* Training on the GPU (no counterpart in the reference): loss = -mean log(4 pi q(n | features)) over samples (maximum likelihood of the site's
  * conditional distribution), Adam (beta 0.9 / 0.999, eps 1e-8) on FP32 master weights, BF16-rounded weights in
- * the passes. Batches are device buffers in the mcl_extract_samples format, at most max_batch rows. */
+ * the passes. Batches are device buffers in the mcl_extract_samples format, at most max_batch rows. They must be
+ * complete when a step or gradient is called, and left alone until it has ended: a trainer works on a stream of its
+ * own, which waits for no other. */
 typedef struct mcl_trainer mcl_trainer;
 int mcl_trainer_create(const mcl_mlp *init, long long max_batch, float kappa_max, mcl_trainer **out);
 /* Gradient of the mean loss at the current weights (no update) and the loss. Synchronises. */

@@ -43,6 +43,8 @@ def collect(engine, snapshots, gap, per_snapshot, seed=3, replicas=None):
     n = snapshots * len(reps) * per_snapshot
     feat = torch.empty((n, 8), dtype=torch.float32, device="cuda")
     dirs = torch.empty((n, 3), dtype=torch.float32, device="cuda")
+    # the engine's stream is not torch's, on which work with memory now reused may still be queued
+    torch.cuda.current_stream().synchronize()
     k = 0
     for s in range(snapshots):
         engine.sweeps(gap)
@@ -73,6 +75,7 @@ def train(feat, dirs, epochs=3, batch=8192, lr=3e-3, lr_end=1e-4, seed=3, params
                 fb, db = feat[idx].contiguous(), dirs[idx].contiguous()
                 step = ep * per_epoch + i
                 rate = lr_end + 0.5 * (lr - lr_end) * (1 + math.cos(math.pi * step / max(1, total - 1)))
+                torch.cuda.current_stream().synchronize()  # the trainer's stream does not wait for the gathers
                 losses.append(t.step(fb.data_ptr(), db.data_ptr(), batch, rate))
         out = t.params()
     finally:
