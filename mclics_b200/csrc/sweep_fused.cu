@@ -425,7 +425,7 @@ static int clusters_that_fit(const mcl_engine *e, int C) {
   l.max_clusters = &fit;
   if (resident_dispatch(e, ResidentArgs{}, l) != cudaSuccess) {
     cudaGetLastError();
-    fit = 0;
+    return 0;
   }
   known[{e->device, C}] = fit;
   return fit;
@@ -454,13 +454,9 @@ static void resident_choose(const mcl_engine *e, FusedPlan *P) {
   int min_nz = 1 << 30, sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
   for (const auto &D : e->desc) min_nz = std::min(min_nz, D.nz);
-  ResidentLaunch limits = resident_desc(e, 1, 0);
-  limits.prepare = true;
-  if (resident_dispatch(e, ResidentArgs{}, limits) != cudaSuccess) {
-    cudaGetLastError();  // this combination of options has no kernel
-    return;
-  }
   if (P->C.kind != 1) return;
+  // Setting the kernel's limits loads it, which takes milliseconds: not before a replica fits and could be faster.
+  bool prepared = false;
   const double pass = 5.0 + 2.0 * pass_time(e, P->cfg, P->seg, sms);  // the finalisation and the gaps between launches
   double best = pass;
   for (int C = 1; C <= kResMaxC && C <= min_nz; C *= 2) {
@@ -468,16 +464,31 @@ static void resident_choose(const mcl_engine *e, FusedPlan *P) {
     for (const auto &D : e->desc)
       smem = std::max(smem, kResHead + ((size_t)(D.nz + C - 1) / C + 2) * res_plane(D.nx, D.ny) * sizeof(float));
     if (smem > kResMaxSmem) continue;
+    auto alone = [&](const RepDesc &D) {  // one sweep of a replica
+      const double tasks = std::ceil((double)D.nz / C) * D.ny * res_pairs(D.nx);
+      return 2.0 * (std::max(0.8, round * tasks / kResThreads) + 0.4 + 0.08 * C);
+    };
+    double cost = 0;
+    for (const auto &D : e->desc) cost = std::max(cost, alone(D));
+    if (1.1 * cost + 3.0 >= best) continue;  // all replicas at once
+    if (!prepared) {
+      ResidentLaunch limits = resident_desc(e, 1, 0);
+      limits.prepare = true;
+      if (resident_dispatch(e, ResidentArgs{}, limits) != cudaSuccess) {
+        cudaGetLastError();  // this combination of options has no kernel
+        return;
+      }
+      prepared = true;
+    }
     const int fit = clusters_that_fit(e, C);
     if (fit < 1) continue;
     // replicas in order onto the cluster that is free first
     std::vector<double> busy((size_t)std::min(fit, e->n_rep), 0.0);
     std::make_heap(busy.begin(), busy.end(), std::greater<double>());
-    double cost = 0;
+    cost = 0;
     for (const auto &D : e->desc) {
-      const double tasks = std::ceil((double)D.nz / C) * D.ny * res_pairs(D.nx);
       std::pop_heap(busy.begin(), busy.end(), std::greater<double>());
-      busy.back() += 2.0 * (std::max(0.8, round * tasks / kResThreads) + 0.4 + 0.08 * C);
+      busy.back() += alone(D);
       cost = std::max(cost, busy.back());
       std::push_heap(busy.begin(), busy.end(), std::greater<double>());
     }
