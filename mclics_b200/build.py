@@ -22,9 +22,16 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-O3", "--expt-relaxed-constexpr",
           "-I" + os.path.join(HERE, "..", "include")] + ARCH
 PER_FILE = {"kernels_ref8.cu": ["-fmad=false"]}
-SOURCES = ["sweep_pass_ghrl.cu", "sweep_pass_ghrl_chiral.cu", "sweep_pass_pear.cu", "sweep_pass_ll.cu",
-           "sweep_resident_ghrl.cu", "sweep_resident_ghrl_chiral.cu", "sweep_resident_pear.cu", "sweep_resident_ll.cu",
-           "sweep_fused_ghrl.cu", "sweep_fused_pear.cu", "sweep_fused_ll.cu", "learned.cu", "kernels.cu",
+# Sources compiled once per set of macros: {file: {object suffix: flags}}.
+VARIANTS = {"sweep_pass_kernels.cu": {
+    "%s%s%s%s" % (pot, "_chiral" * chiral, "_flip" * flip, "_field" * field):
+        ["-DPASS_POT=POT_" + pot.upper()] + ["-DPASS_%s=%s" % (k, str(bool(v)).lower())
+                                             for k, v in (("CHIRAL", chiral), ("FLIP", flip), ("FIELD", field))]
+    for pot, chiral, flip, field in (("ghrl", 1, 1, 1), ("ghrl", 1, 0, 1), ("ghrl", 1, 0, 0), ("ghrl", 0, 1, 1),
+                                     ("ghrl", 0, 0, 1), ("ghrl", 0, 0, 0), ("pear", 0, 1, 1), ("pear", 0, 1, 0),
+                                     ("ll", 0, 1, 1), ("ll", 0, 0, 1), ("ll", 0, 0, 0))}}
+SOURCES = ["sweep_pass_kernels.cu", "sweep_pass.cu", "sweep_resident_ghrl.cu", "sweep_resident_ghrl_chiral.cu",
+           "sweep_resident_pear.cu", "sweep_resident_ll.cu", "sweep_fused_ghrl.cu", "sweep_fused_pear.cu", "sweep_fused_ll.cu", "learned.cu", "kernels.cu",
            "kernels_ref8.cu", "sweep_fused.cu", "observe_static.cu", "extras.cu", "engine.cpp", "driver.cpp"]  # slowest first: they start compiling first
 
 
@@ -44,12 +51,23 @@ def _deps_newer(obj, src):
     return any(os.path.getmtime(p) > t for p in [src] + heads)
 
 
-def _compile(src, verbose):
+def _units():
+    """(source, flags, object) of everything that is compiled."""
+    out = []
+    for src in SOURCES:
+        if os.path.exists(os.path.join(CSRC, src)):
+            for suffix, flags in VARIANTS.get(src, {"": []}).items():
+                obj = src + ("." + suffix if suffix else "") + ".o"
+                out.append((src, PER_FILE.get(src, []) + flags, os.path.join(BUILD, obj)))
+    return out
+
+
+def _compile(unit, verbose):
+    src, flags, obj = unit
     path = os.path.join(CSRC, src)
-    obj = os.path.join(BUILD, src + ".o")
     if not _deps_newer(obj, path):
         return obj
-    cmd = [nvcc()] + COMMON + PER_FILE.get(src, []) + ["-c", path, "-o", obj]
+    cmd = [nvcc()] + COMMON + flags + ["-c", path, "-o", obj]
     if src.endswith(".cpp"):
         cmd[1:1] = ["-x", "cu"]
     if verbose:
@@ -62,14 +80,13 @@ def _compile(src, verbose):
 
 def build(force=False, verbose=False):
     os.makedirs(BUILD, exist_ok=True)
-    srcs = [s for s in SOURCES if os.path.exists(os.path.join(CSRC, s))]
+    units = _units()
     if force:
-        for s in srcs:
-            p = os.path.join(BUILD, s + ".o")
-            if os.path.exists(p):
-                os.remove(p)
+        for _, _, obj in units:
+            if os.path.exists(obj):
+                os.remove(obj)
     with cf.ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as ex:
-        objs = list(ex.map(lambda s: _compile(s, verbose), srcs))
+        objs = list(ex.map(lambda u: _compile(u, verbose), units))
     if force or not os.path.exists(LIB) or any(os.path.getmtime(o) > os.path.getmtime(LIB) for o in objs):
         cmd = [nvcc()] + ARCH + ["-shared", "-cudart", "static", "-o", LIB] + objs
         r = subprocess.run(cmd, capture_output=True, text=True)
