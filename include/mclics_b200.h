@@ -266,11 +266,13 @@ int mcl_zslab_pack(mcl_engine *e, float *send_lo, float *send_hi);          /* n
 int mcl_zslab_unpack(mcl_engine *e, const float *recv_lo, const float *recv_hi); /* null: no neighbour there */
 int mcl_zslab_sums(mcl_engine *e, int measure, double *d_sums);
 int mcl_zslab_finalize(mcl_engine *e, const double *d_sums, int measure);
-/* With enable != 0, mcl_sweeps (and mcl_sweeps_io) replay a captured CUDA graph of eight sweeps (colour-pass
- * plans) or two (the ping-pong fused plans 0 and 1; what is left over is launched one by one), captured at the first call and again after the plan, the series buffer
- * or the test hooks change, instead of launching kernels one by one; results are identical. Profiling (mcl_profile)
- * uses direct launches. */
+/* With enable != 0, mcl_sweeps (and mcl_sweeps_io) replay captured CUDA graphs: of eight sweeps, or of one for a call
+ * of one sweep (colour-pass plans), or of two (the ping-pong fused plans 0 and 1). What is left over is launched kernel
+ * by kernel. They are captured at the first call and again after the plan, the series buffer or the test hooks change;
+ * results are identical. Profiling (mcl_profile) uses direct launches. */
 int mcl_set_graphs(mcl_engine *e, int enable);
+/* Test hook: graphs of sweeps that this engine has launched so far. */
+int mcl_debug_graph_replays(mcl_engine *e, long long *replays);
 
 /* ---- Learned Metropolis-Hastings proposal (no counterpart in the reference) ----------------------------------
  * Per site, a 7 -> 64 -> 64 -> 4 MLP with SiLU reads the neighbour Q-tensor sum sum_j (3 n_j n_j^T - I)/2 divided by

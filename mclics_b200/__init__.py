@@ -108,6 +108,7 @@ def lib():
             "mcl_measure_extras": [vp, i, P(ctypes.c_double * 3), P(CExtras)],
             "mcl_local_order": [vp, i, vp],
             "mcl_set_graphs": [vp, i],
+            "mcl_debug_graph_replays": [vp, P(ctypes.c_longlong)],
             "mcl_set_plan": [vp, i, i],
             "mcl_zslab_init": [vp, i, i, i, P(ctypes.c_longlong)],
             "mcl_zslab_pass": [vp, i, i],
@@ -353,6 +354,11 @@ class Engine:
 
     def debug_wait_limit(self, timeout_ns, withhold_first_load=False):
         check(lib().mcl_debug_wait_limit(self._h, timeout_ns, 1 if withhold_first_load else 0))
+
+    def debug_graph_replays(self):
+        n = ctypes.c_longlong()
+        check(lib().mcl_debug_graph_replays(self._h, ctypes.byref(n)))
+        return n.value
 
     def record_decisions(self, on=True):
         check(lib().mcl_record_decisions(self._h, 1 if on else 0))

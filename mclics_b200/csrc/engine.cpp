@@ -351,33 +351,32 @@ static int kernel_errors(mcl_engine *e) {
 // Captured sweep graphs hold kernel arguments (work items, buffers, series, test hooks): drop them whenever one of
 // those changes.
 static void drop_graphs(mcl_engine *e) {
-  for (int m = 0; m < 2; m++) {
-    if (e->graph[m]) cudaGraphExecDestroy(e->graph[m]);
-    e->graph[m] = nullptr;
+  for (SweepGraph *g : {&e->graph[0], &e->graph[1], &e->graph_one[0], &e->graph_one[1]}) {
+    if (g->exec) cudaGraphExecDestroy(g->exec);
+    *g = SweepGraph();
   }
-  e->graph_series = nullptr;
   if (e->graph_io) cudaGraphExecDestroy(e->graph_io);
   e->graph_io = nullptr;
   e->graph_io_series = e->graph_io_stage = nullptr;
 }
 
-// Sweeps per captured graph: eight for the in-place colour passes (kernels overlap at their ends inside a graph, not
-// between two graphs), two for the ping-pong fused kernel (one per buffer parity, so that a replay leaves the buffers
+// Sweeps per captured graph of a longer call: eight for the in-place colour passes (kernels overlap at their ends inside
+// a graph, not between two graphs), two for the ping-pong fused kernel (one per buffer parity, so that a replay leaves the buffers
 // where it found them).
 static int graph_sweeps(const mcl_engine *e) { return fused_is_pass_plan(e) ? 8 : 2; }
 
-// Captures graph_sweeps(e) sweeps starting from buffer e->cur as a graph. Every per-sweep quantity the kernels use
-// (sweep counter, temperatures, ang_var, series length) lives in device memory, so a replay does exactly what the
-// same direct calls would.
-static int capture_graph(mcl_engine *e, int m) {
-  if (e->graph[m]) cudaGraphExecDestroy(e->graph[m]);
-  e->graph[m] = nullptr;
+// Captures `sweeps` sweeps starting from buffer e->cur as a graph. Every per-sweep quantity the kernels use (sweep
+// counter, temperatures, ang_var, series length) lives in device memory, so a replay does exactly what the same direct
+// calls would.
+static int capture_graph(mcl_engine *e, SweepGraph &sg, int sweeps, bool measure) {
+  if (sg.exec) cudaGraphExecDestroy(sg.exec);
+  sg = SweepGraph();
   cudaGraph_t g = nullptr;
   CK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
   const int cur0 = e->cur;
   const long long l0 = e->launches;
   int rc = MCL_OK;
-  for (int s = 0; s < graph_sweeps(e) && !rc; s++) rc = fused_sweep(e, m != 0, nullptr, nullptr);
+  for (int s = 0; s < sweeps && !rc; s++) rc = fused_sweep(e, measure, nullptr, nullptr);
   const cudaError_t ce = cudaStreamEndCapture(e->stream, &g);
   e->cur = cur0;
   e->launches = l0;
@@ -386,14 +385,15 @@ static int capture_graph(mcl_engine *e, int m) {
     return rc;
   }
   if (ce != cudaSuccess) return cuda_fail(ce, "cudaStreamEndCapture");
-  const cudaError_t ie = cudaGraphInstantiate(&e->graph[m], g, 0);
+  const cudaError_t ie = cudaGraphInstantiate(&sg.exec, g, 0);
   cudaGraphDestroy(g);
   if (ie != cudaSuccess) {
-    e->graph[m] = nullptr;
+    sg.exec = nullptr;
     return cuda_fail(ie, "cudaGraphInstantiate");
   }
-  e->graph_cur[m] = cur0;
-  if (m) e->graph_series = e->d_series;
+  sg.sweeps = sweeps;
+  sg.cur = cur0;
+  if (measure) sg.series = e->d_series;
   return MCL_OK;
 }
 
@@ -862,6 +862,20 @@ static int profile_events(mcl_engine *e, int sweeps, cudaEvent_t *ev0, cudaEvent
   return MCL_OK;
 }
 
+// Whether the caller is capturing the engine's stream, and whether nothing is queued on it.
+static bool capturing(const mcl_engine *e) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(e->stream, &s) == cudaSuccess) return s != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;
+}
+static bool idle(const mcl_engine *e) {
+  if (capturing(e)) return false;  // which a query would end
+  if (cudaStreamQuery(e->stream) == cudaSuccess) return true;
+  cudaGetLastError();
+  return false;
+}
+
 static int sweeps_run(mcl_engine *e, int n, int measure) {
   int rc;
   if (measure && (rc = ensure_series(e, e->series_len + n))) return rc;
@@ -871,9 +885,7 @@ static int sweeps_run(mcl_engine *e, int n, int measure) {
   // would keep the lists of a geometry that may have been replaced when it is replayed.
   bool by_lists = e->geo == GEO_PT && e->schedule == MCL_SCHED_CHECKER2 && !e->record_dec;
   if (by_lists) {
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    CK(cudaStreamIsCapturing(e->stream, &capture));
-    by_lists = capture == cudaStreamCaptureStatusNone;
+    by_lists = !capturing(e);
     if (by_lists && e->pt_lists_stale && (rc = build_pt_lists(e))) return rc;
     by_lists = by_lists && e->pt_lists.n_blocks > 0;
   }
@@ -892,19 +904,26 @@ static int sweeps_run(mcl_engine *e, int n, int measure) {
     }
     return MCL_OK;
   }
-  const int per_graph = use_fused ? graph_sweeps(e) : 2;
-  if (use_fused && e->use_graphs && !e->profile && n >= per_graph) {
+  // A call of one sweep on an idle stream has a graph of its own, as three launches would follow one another from the
+  // host (LL 64^3 and a wait 52.0 -> 50.3 us, 32^3 on plan 4 37.2 -> 34.9); on a busy stream launches overlap the sweep
+  // before, which graphs do not (29.0 against 31.2 us).
+  const bool graphs = use_fused && e->use_graphs && !e->profile;
+  const bool lone = graphs && n == 1 && fused_is_pass_plan(e) && idle(e);
+  const int per_graph = lone ? 1 : graph_sweeps(e);
+  if (graphs && n >= per_graph) {
     const int m = measure ? 1 : 0;
-    if (!e->graph[m] || (m && e->graph_series != (const void *)e->d_series)) {
-      if ((rc = capture_graph(e, m))) return rc;
+    SweepGraph &g = per_graph == 1 ? e->graph_one[m] : e->graph[m];
+    if (!g.exec || g.sweeps != per_graph || (m && g.series != (const void *)e->d_series)) {
+      if ((rc = capture_graph(e, g, per_graph, measure != 0))) return rc;
     }
-    if (e->cur != e->graph_cur[m]) {  // one direct sweep brings the buffers to the graph's parity
+    if (e->cur != g.cur) {  // one direct sweep brings the buffers to the graph's parity
       if ((rc = fused_sweep(e, measure != 0, nullptr, nullptr))) return rc;
       if (measure) e->series_len++;
       n--;
     }
     for (; n >= per_graph; n -= per_graph) {
-      CK(cudaGraphLaunch(e->graph[m], e->stream));
+      CK(cudaGraphLaunch(g.exec, e->stream));
+      e->graph_replays++;
       e->launches += per_graph * fused_launches_per_sweep(e);
       if (measure) e->series_len += per_graph;
     }
@@ -1045,6 +1064,7 @@ int mcl_sweeps_io(mcl_engine *e, int n, const float *T, mcl_observables *out) {
     memcpy(hT, T, (size_t)e->n_rep * sizeof(float));
     e->io_inflight = true;
     CK(cudaGraphLaunch(e->graph_io, e->stream));
+    e->graph_replays++;
     e->launches += 2 + (resident ? 1 : fused_launches_per_sweep(e));
     e->series_len++;
   } else {
@@ -1193,6 +1213,12 @@ int mcl_debug_wait_limit(mcl_engine *e, long long timeout_ns, int withhold_first
   drop_graphs(e);
   if (!e->fused) return fail(MCL_ERR_STATE, "this engine does not use the fused tiled sweep");
   fused_set_test_hooks(e, timeout_ns, withhold_first_load);
+  return MCL_OK;
+}
+
+int mcl_debug_graph_replays(mcl_engine *e, long long *replays) {
+  if (!e || !replays) return fail(MCL_ERR_ARG, "null argument");
+  *replays = e->graph_replays;
   return MCL_OK;
 }
 

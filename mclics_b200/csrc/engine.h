@@ -28,6 +28,12 @@ constexpr int kCopySlots = 8;
 int copy_out(mcl_engine *e, void *dst, const void *d_src, size_t bytes);
 
 struct FusedPlan;  // fused tiled sweep (sweep_fused.cu)
+// A captured graph of sweeps: the director buffer it starts from and the series buffer it writes (if it measures).
+struct SweepGraph {
+  cudaGraphExec_t exec = nullptr;
+  int sweeps = 0, cur = 0;
+  const void *series = nullptr;
+};
 struct MlpDev;     // learned proposal weights in device layout (learned.cu)
 struct MlpTC;      // the same in the tcgen05 layout (mlp_tc.cuh)
 int learned_check_error(mcl_engine *e);
@@ -95,10 +101,9 @@ struct mcl_engine {
   bool adapt = true;           // ang_var adaptation after each sweep (the reference's behaviour)
   int mix_period = 1;          // with a learned proposal: every mix_period-th sweep learned, the others plain
   int mix_phase = 0;           // sweeps since the last learned one (mcl_set_proposal_mix)
-  bool use_graphs = false;     // fused sweeps replayed from captured CUDA graphs (one or two sweeps each)
-  cudaGraphExec_t graph[2] = {nullptr, nullptr};  // [measure]: the sweeps of one replay, from buffer graph_cur
-  int graph_cur[2] = {0, 0};
-  const void *graph_series = nullptr;             // series buffer the measuring graph writes
+  bool use_graphs = false;     // sweeps replayed from captured CUDA graphs (graph_sweeps of them, or one)
+  mcl::SweepGraph graph[2], graph_one[2];  // [measure]: several sweeps (graph_sweeps), and a single one
+  long long graph_replays = 0;  // sweep graphs launched so far
   cudaGraphExec_t graph_io = nullptr;  // mcl_sweeps_io's step (input kernel, one measured sweep, output kernel)
   const void *graph_io_series = nullptr, *graph_io_stage = nullptr;  // the buffers it was captured with
   cudaStream_t copy_stream = nullptr;  // of large device-to-host copies (copy_out)
