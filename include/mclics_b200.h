@@ -170,7 +170,8 @@ int mcl_read_decisions(mcl_engine *e, int replica, unsigned char *out);
  * reference uses the default stream). */
 int mcl_set_stream(mcl_engine *e, void *stream);
 /* Kernel timing: with enable != 0 every following sweep records CUDA events around its sweep kernel(s) (not the
- * per-sweep finalisation); mcl_profile_read returns their total time in ms and the number of sweeps timed, and
+ * per-sweep finalisation, except that the resident sweep of small lattices has it inside its one launch, whose time
+ * counts for all its sweeps); mcl_profile_read returns their total time in ms and the number of sweeps timed, and
  * the number of kernels this engine has launched since creation. No counterpart in the reference. */
 int mcl_profile(mcl_engine *e, int enable);
 int mcl_profile_read(mcl_engine *e, double *sweep_kernel_ms, long long *timed_sweeps, long long *kernel_launches);
@@ -220,7 +221,11 @@ int mcl_local_order(mcl_engine *e, int replica, float *S);
  * choice to the engine where it is the fastest; the plan fields of *out are then those of the fastest colour-pass plan,
  * which shorter calls run.
  * The fused configurations need a second director buffer, allocated while one of them is selected and freed when a
- * colour-pass configuration is selected again. Every configuration gives bit-identical directors. Candidate plans:
+ * colour-pass configuration is selected again. Every configuration gives bit-identical directors, with one exception:
+ * on a Lebwohl-Lasher bulk lattice without a field the colour passes and the resident sweep round a trial's energy
+ * difference once, while the fused configurations, the untiled kernel and the colour-1 half of a measured sweep round
+ * it twice. A trial within that rounding of its threshold (at T = 0 a neutral one too) may then be decided either way,
+ * so that a fused plan or not, and measuring or not, are different chains of the same distribution. Candidate plans:
  * per configuration the heuristic segment length, its double, its half and the whole depth; lattices that give
  * fewer work items than SMs also 2-4 planes in the colour passes. mcl_autotune times each candidate plan for
  * trial_sweeps measured sweeps on the engine's own replicas, keeps the fastest and restores the directors,

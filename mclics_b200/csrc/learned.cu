@@ -737,8 +737,8 @@ __device__ __forceinline__ void tile_product(const float (*a)[kTP], const float 
 //
 // Bound by the FP32 pipe in its three 64 x 64 x 64 products (115 M multiply-adds for 8192 samples: 3 us over the chip)
 // and the latency of its phases. One thread per sample, 64 per block, it ran at 3 % of the warps and one shared load per
-// multiplication (55 us); 256 threads with 4 x 4 register tiles take 22 us. Every sum keeps its order of terms, so
-// gradients are the same bits.
+// multiplication (55 us); 256 threads with 4 x 4 register tiles take 22 us. Every sum of a block keeps its order of terms,
+// so its partial gradients are the same bits; the FP64 sum over the blocks (k_grad_reduce) is grouped by warps.
 __global__ void __launch_bounds__(kTT) k_mlp_grad(const float *__restrict__ wr, const float *__restrict__ feat,
                                                   const float *__restrict__ dirs, long long n, float kappa_max,
                                                   float scale, float *__restrict__ partial) {

@@ -451,7 +451,9 @@ __device__ __forceinline__ V3<L> sel3(LB<L> c, const V3<L> &a, const V3<L> &b) {
 // Compile-time features: FLIP (n -> -n trial), PRES (neighbours always present), CHIRAL (GHRL sigma term),
 // FIELD (field term), SINGLE = false (the caller knows the site has no single-site term: no surface, no field;
 // the energies are then the bond sums themselves, which is what adding the zero single term gives, up to the sign
-// of a zero). Every combination rounds like the general one on the inputs it applies to.
+// of a zero). Every combination rounds like the general one on the inputs it applies to, except FUSED (Lebwohl-Lasher
+// only), which rounds the energy difference once instead of twice. Unmeasured bulk passes without a field have always
+// been that way, first by the compiler's contraction; the other callers never were, and either form keeps its chains.
 template <int POT, bool FLIP, int PRES, int CHIRAL, bool FIELD, typename L, bool SINGLE = true, bool FUSED = false>
 __device__ __forceinline__ SiteResultT<L> site_update(const ModelDev &m, const V3<L> &n, const V3<L> (&nb)[6],
                                                       const L (&w)[6], int sid, const Vec3 &s, float elecE,

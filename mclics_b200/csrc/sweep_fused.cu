@@ -434,17 +434,17 @@ static int clusters_that_fit(const mcl_engine *e, int C) {
 // CTAs per replica of the resident kernel, or 0 where the colour passes are faster or a replica does not fit.
 //
 // Measured per sweep on one B200 (us, unmeasured / measured sweeps in long calls; colour passes on their best plan with
-// graph replay):
-//                     resident, C = 4     C = 8          C = 16         colour passes
-//   LL 16^3           3.6 / 4.5           3.2 / 4.0      3.5 / 4.2      14.4 / 16.5
-//   LL 32^3           12.9 / 14.3         7.8 / 8.5      6.7 / 6.9      14.4 / 16.5
-//   LL 48^3           does not fit        does not fit   12.8 / 13.6    14.4 / 18.6
-//   GHRL 32^3         16.4 / 17.6         9.5 / 10.1     7.6 / 7.8      14.4 / 16.5
-//   chiral 32^3       20.2 / 21.7         11.5 / 12.2    8.6 / 8.8      14.4 / 18.4
-//   pear 48 x 48 x 24 41 / 45             23.6 / 25.4    18.0 / 19.7    24.7 / 26.9
-//   LL 32 x 32^3      13.2 / 16.8         23.3 / 27.9    32.4 / 37.2    26.8 / 30.8
-//   LL 64 x 24^3      15.1 / 18.4         25.4 / 30.2    44.2 / 74.9    37.5 / 41.0
-//   LL 128 x 16^3     14.4 / 20.0         28.0 / 40.5    62.6 / 86.9    30.8 / 33.0
+// graph replay; the resident kernel as chosen here where it is):
+//                     resident, C = 4     C = 8          C = 16         chosen         colour passes
+//   LL 16^3           3.6 / 4.5           3.2 / 4.0      3.5 / 4.2      3.6 / 4.4      10.5 / 12.8
+//   LL 32^3           12.9 / 14.3         7.8 / 8.5      6.7 / 6.9      6.6 / 6.7      10.8 / 12.7
+//   LL 48^3           does not fit        does not fit   12.8 / 13.6    -              12.0 / 14.9
+//   GHRL 32^3         16.4 / 17.6         9.5 / 10.1     7.6 / 7.8      7.5 / 7.6      11.3 / 13.3
+//   chiral 32^3       20.2 / 21.7         11.5 / 12.2    8.6 / 8.8      8.2 / 8.3      11.6 / 14.0
+//   pear 48 x 48 x 24 41 / 45             23.6 / 25.4    18.0 / 19.7    -              16.4 / 20.8
+//   LL 32 x 32^3      13.2 / 16.8         23.3 / 27.9    32.4 / 37.2    13.0 / 14.2    24.4 / 27.5
+//   LL 64 x 24^3      15.1 / 18.4         25.4 / 30.2    44.2 / 74.9    12.9 / 13.8    38.6 / 41.8
+//   LL 128 x 16^3     14.4 / 20.0         28.0 / 40.5    62.6 / 86.9    7.3 / 8.2      28.0 / 31.7
 // A colour costs a chain of one task or the issue of the tasks of a full CTA, `round` us per 512, and a cluster barrier
 // that grows with C; replicas beyond the clusters that fit the device (33, 15 and 7) wait for a free one.
 static void resident_choose(const mcl_engine *e, FusedPlan *P) {

@@ -5,7 +5,7 @@
 // same launch writes, and can write its sites back into the buffer it reads: no second buffer, no recomputed ring,
 // no halo planes computed twice. A sweep is two passes (colour 0 = x + y + z even, then colour 1), each exactly
 // one site update per owned site; the results are bit-identical to the fused kernel's (same draws, same arithmetic,
-// same order of colours).
+// same order of colours), but for the rounding named at site_update (physics.cuh, FUSED).
 //
 // Work item = (replica, TX x TY tile, z segment [z0, z1)). The CTA streams planes z0 - 1 .. z1 through NSLP = 4
 // shared-memory slots; each slot is one 5-D TMA box (TX / 2 + 8 half-row cells, 2 parities, TY + 2 rows, 1 plane,

@@ -1,8 +1,8 @@
 // Resident sweep: small bulk and slab lattices swept entirely in shared memory, any number of sweeps in one launch.
 //
 // A 32^3 lattice is 393 KB: the colour passes (sweep_pass.cuh) give it 10-32 work items, and a sweep costs three
-// dependent launches whose chains of plane loads leave the chip idle (22-38 us for a measured sweep of 32^3, of which
-// under 1 us is work). Here one thread-block cluster holds a replica: CTA c of C keeps the planes
+// dependent launches whose chains of plane loads leave the chip idle (13-28 us for a measured sweep of 32^3 by plan, of
+// which under 1 us is work). Here one thread-block cluster holds a replica: CTA c of C keeps the planes
 // [c nz / C, (c + 1) nz / C) and a copy of the two planes next to them, and all sweeps of a call run without leaving
 // the kernel. Per colour, a task is the same pair of sites (x, x + 2) with the same draws and the same site_update as
 // in the colour passes, so directors, acceptances and amplitudes are the same bits. Its sites of the first or last
@@ -11,8 +11,9 @@
 //
 // Bound by the instruction issue of the C <= 16 SMs a replica occupies (1.45 us per colour for one LL pair per thread)
 // and by the latency of one task and one cluster barrier (1.6 us per colour at least). LL 32^3 per sweep of a long call:
-// 6.7 us, measured 6.9 (three launches on the best colour-pass plan: 14.4, 16.5; on the default one 28.8, 31.1);
-// 32 such replicas 13.2, 16.8 (26.8, 30.8). resident_choose (sweep_fused.cu) has both sides over the sizes.
+// 6.6 us, measured 6.7 (three launches on the best colour-pass plan, replayed from graphs: 10.8, 12.7); 32 such replicas
+// 13.0, 14.2 (24.4, 27.5). resident_choose (sweep_fused.cu) has both sides over the sizes. Counters: 332 (measured 384)
+// instructions per site update at 40-46 % issue of the 16 SMs it runs on.
 //
 // Planes in shared memory: [plane][component][y][x parity][cell], cells of a half-row as in HBM (common.cuh) with two
 // cells of padding left and right, which hold the periodic x ghosts; periodic y is an address, periodic z the copies.
