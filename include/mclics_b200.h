@@ -114,7 +114,7 @@ int mcl_set_geometry(mcl_engine *e, int replica, const int *pt, const float *nor
 int mcl_upload_directors(mcl_engine *e, int replica, const float *ni);
 int mcl_download_directors(mcl_engine *e, int replica, float *ni);
 /* Downloads of 16 MiB and more (directors, local order) pass through pinned memory that the library keeps for the next
- * one, of any engine: at most 8 MiB per process. mcl_trim gives back what no download is using. */
+ * one, of any engine: at most 12 MiB per process. mcl_trim gives back what no download is using. */
 int mcl_trim(void);
 
 /* Random initial condition of one replica on the device (replaces the host loop of `ic random`,

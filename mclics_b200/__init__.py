@@ -496,7 +496,7 @@ class Trainer:
 
 
 def trim():
-    """Gives back the pinned memory kept between large downloads (at most 8 MiB per process)."""
+    """Gives back the pinned memory kept between large downloads (at most 12 MiB per process)."""
     check(lib().mcl_trim())
 
 

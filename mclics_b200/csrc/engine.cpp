@@ -87,10 +87,12 @@ static void sphere_geometry(int nx, int ny, int nz, int *pt, float *ns) {
 // hands out memory that is already mapped, a plain copy is as fast (0.76 against 0.92 ms for 12.6 MB).
 //
 // Pinning a ring takes 3-4 ms, so rings belong to the process, at most kRings of them, and any engine takes a free one
-// (none free: a plain copy). First download of a new engine, in ms (plain copy; a ring of its own; a ring that is there):
+// (none free: a plain copy). They are taken in turn, because the device writes faster to slots that no core has in its
+// cache any more (local order of 256 x 256 x 64 after the field: 0.95 ms, 1.25 with one ring); another one is pinned
+// every kCopiesPerRing copies. First download of a new engine, in ms (plain copy; a ring of its own; a ring that is there):
 // 25 MB 2.5, 7.0, 1.5; 50 MB 10.4, 9.7, 4.3; 201 MB 41, 20, 13.5. The first large copy of all makes a ring only from
 // kRingWorthPinning on: below it the pinning costs what a plain copy does (25 MB into a fresh array: 7 and 5-8 ms).
-constexpr int kRings = 2;
+constexpr int kRings = 3, kCopiesPerRing = 4;
 constexpr size_t kCopyChunk = 512 << 10, kCopyLarge = 16 << 20, kRingWorthPinning = 32 << 20;
 
 // Whether host memory is pinned already: the device writes to it directly, a 201 MB field in 3.8 ms (9.1 through a ring).
@@ -106,7 +108,8 @@ struct RingPool {
   std::mutex mu;
   char *ring[kRings] = {};
   bool busy[kRings] = {};
-  long long asked = 0;  // large copies so far
+  long long last[kRings] = {};  // the copy that used it last
+  long long copies = 0;         // large copies so far
 } g_rings;
 
 // A ring for the time of one copy of `bytes`: slots() is null when there is none to be had.
@@ -114,20 +117,24 @@ class RingLease {
  public:
   explicit RingLease(size_t bytes) {
     std::lock_guard<std::mutex> lock(g_rings.mu);
-    const bool pin = g_rings.asked++ > 0 || bytes >= kRingWorthPinning;
-    for (int i = 0; i < kRings && id_ < 0; i++)
-      if (!g_rings.busy[i] && alive(i)) id_ = i;
-    for (int i = 0; i < kRings && id_ < 0 && pin; i++)
-      if (!g_rings.busy[i]) {
-        if (cudaHostAlloc((void **)&g_rings.ring[i], kCopySlots * kCopyChunk, cudaHostAllocPortable) == cudaSuccess)
-          id_ = i;
-        else {
-          cudaGetLastError();
-          g_rings.ring[i] = nullptr;
-        }
-        break;
-      }
-    if (id_ >= 0) g_rings.busy[id_] = true;
+    const long long n = ++g_rings.copies;
+    int oldest = -1, none = -1, rings = 0;
+    for (int i = 0; i < kRings; i++) {
+      const bool there = g_rings.busy[i] || alive(i);
+      rings += there;
+      if (!there) none = i;
+      if (there && !g_rings.busy[i] && (oldest < 0 || g_rings.last[i] < g_rings.last[oldest])) oldest = i;
+    }
+    const bool pin = rings == 0 ? n > 1 || bytes >= kRingWorthPinning : oldest < 0 || n > kCopiesPerRing * rings;
+    if (pin && none >= 0 &&
+        cudaHostAlloc((void **)&g_rings.ring[none], kCopySlots * kCopyChunk, cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      g_rings.ring[none] = nullptr;
+    }
+    id_ = pin && none >= 0 && g_rings.ring[none] ? none : oldest;
+    if (id_ < 0) return;
+    g_rings.busy[id_] = true;
+    g_rings.last[id_] = n;
   }
   ~RingLease() {
     if (id_ < 0) return;
@@ -1104,7 +1111,7 @@ int mcl_trim(void) {
       cudaFreeHost(g_rings.ring[i]);
       g_rings.ring[i] = nullptr;
     }
-  g_rings.asked = 0;
+  g_rings.copies = 0;
   return MCL_OK;
 }
 
