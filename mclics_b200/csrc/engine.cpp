@@ -348,6 +348,7 @@ static int build_pt_lists(mcl_engine *e) {
   CK(copy_in(e->stream, t.sites, sites.data(), sites.size() * sizeof(PtSite)));
   CK(copy_in(e->stream, t.blocks, blocks.data(), blocks.size() * sizeof(PtBlock)));
   CK(copy_in(e->stream, t.first, first.data(), first.size() * sizeof(int)));
+  CK(cudaStreamSynchronize(e->stream));
   t.n_blocks = (int)blocks.size();
   return MCL_OK;
 }
@@ -1429,6 +1430,7 @@ int mcl_zslab_init(mcl_engine *e, int nz_global, int z_offset, int periodic_z, l
   D.periodic[2] = periodic_z ? 1 : 0;
   D.n_valid = (double)D.nx * D.ny * nz_global;
   CK(copy_in(e->stream, e->d_desc, &D, sizeof D));
+  CK(cudaStreamSynchronize(e->stream));
   e->zslab = true;
   drop_graphs(e);
   const bool flip = e->model.flip != 0 || e->model.potential == POT_PEAR;

@@ -16,11 +16,11 @@ namespace mcl {
 // Sets the thread's last error message and returns code.
 int fail(int code, const char *fmt, ...);
 int cuda_fail(cudaError_t err, const char *what);
-// Host memory that a set-up prepared, to the device, complete on return. On the stream whose kernels read it: the
-// library's streams do not wait for the default stream, whose copies from pageable memory may return before they end.
+// Pageable host memory that a set-up prepared, to the device. On the stream whose kernels read it: the library's streams
+// do not wait for the default stream, whose copies from pageable memory may return before they end. The driver has
+// staged the source on return; whoever copies waits for the stream once, at the end of the set-up.
 inline cudaError_t copy_in(cudaStream_t stream, void *d_dst, const void *src, size_t bytes) {
-  const cudaError_t err = cudaMemcpyAsync(d_dst, src, bytes, cudaMemcpyHostToDevice, stream);
-  return err != cudaSuccess ? err : cudaStreamSynchronize(stream);
+  return cudaMemcpyAsync(d_dst, src, bytes, cudaMemcpyHostToDevice, stream);
 }
 // Device memory to a caller's pageable memory on the engine's stream; returns when it has arrived. Large copies go
 // through a ring of kCopySlots pinned chunks.

@@ -1383,6 +1383,7 @@ int mcl_set_proposal(mcl_engine *e, const mcl_mlp *mlp, float kappa_max) {
   }
   CKL(copy_in(e->stream, e->d_mlp, &h, sizeof h));
   CKL(copy_in(e->stream, e->d_mlp_tc, &ht, sizeof ht));
+  CKL(cudaStreamSynchronize(e->stream));
   e->kappa_max = kappa_max;
   // tcgen05 unless MCL_LEARNED_MLP=mma selects the mma.sync warps (same network, same rounding points)
   const char *path = getenv("MCL_LEARNED_MLP");

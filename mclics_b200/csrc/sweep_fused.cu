@@ -253,6 +253,7 @@ static int build_items(mcl_engine *e, FusedPlan *P) {
   CKF(cudaMalloc(&P->d_first, first.size() * sizeof(int)));
   CKF(copy_in(e->stream, P->d_first, first.data(), first.size() * sizeof(int)));
   CKF(cudaMalloc(&P->d_partials, (size_t)P->n_items * kPartials * sizeof(double)));
+  CKF(cudaStreamSynchronize(e->stream));
   const bool pass = P->C.kind == 1;
   const int nsl = pass ? NSLP : NSL;
   const size_t slot_floats = ((size_t)3 * (P->tx + 16) * (P->ty + (pass ? 2 : 4)) + 31) / 32 * 32;
