@@ -1259,9 +1259,13 @@ int mcl_autotune(mcl_engine *e, int trial_sweeps, mcl_tuning *out) {
   int rc;
   // where the resident kernel can run it is a candidate, timed over calls long enough for it: at four times the length
   // from which it is chosen, most of what it gains on long calls shows
-  const int res_calls = fused_resident_calls(e);
-  const int res_sweeps = std::max(trial_sweeps, (int)std::min(10000ll, 4ll * res_calls));
-  if ((rc = ensure_series(e, e->series_len + res_sweeps + std::max(1, res_calls)))) return rc;
+  // (the records of that are kept to 64 MB; if there is no room for them it is no candidate)
+  int res_calls = fused_resident_calls(e);
+  const long long room = (64ll << 20) / ((long long)sizeof(ObsRecord) * e->n_rep);
+  const long long long_call = std::max<long long>(res_calls, std::min(4ll * res_calls, room));
+  const int res_sweeps = std::max(trial_sweeps, (int)std::min(10000ll, long_call));
+  if (res_calls && ensure_series(e, e->series_len + res_sweeps + res_calls)) res_calls = 0;
+  if ((rc = ensure_series(e, e->series_len + trial_sweeps + 1))) return rc;
   CK(cudaStreamSynchronize(e->stream));
   // state to restore: directors (with ghosts), per-replica state, sweep counter, series length
   float *save = nullptr;
