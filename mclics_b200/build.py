@@ -31,8 +31,9 @@ VARIANTS = {"sweep_pass_kernels.cu": {
                                      ("ghrl", 0, 0, 1), ("ghrl", 0, 0, 0), ("pear", 0, 1, 1), ("pear", 0, 1, 0),
                                      ("ll", 0, 1, 1), ("ll", 0, 0, 1), ("ll", 0, 0, 0))}}
 SOURCES = ["sweep_pass_kernels.cu", "sweep_pass.cu", "sweep_resident_ghrl.cu", "sweep_resident_ghrl_chiral.cu",
-           "sweep_resident_pear.cu", "sweep_resident_ll.cu", "sweep_fused_ghrl.cu", "sweep_fused_pear.cu", "sweep_fused_ll.cu", "learned.cu", "kernels.cu",
-           "kernels_ref8.cu", "sweep_fused.cu", "observe_static.cu", "extras.cu", "engine.cpp", "driver.cpp"]  # slowest first: they start compiling first
+           "sweep_resident_pear.cu", "sweep_resident_ll.cu", "sweep_fused_ghrl.cu", "sweep_fused_pear.cu",
+           "sweep_fused_ll.cu", "learned.cu", "kernels.cu", "kernels_ref8.cu", "sweep_fused.cu", "observe_static.cu",
+           "extras.cu", "engine.cpp", "driver.cpp"]  # slowest first: they start compiling first
 
 
 def nvcc():
