@@ -258,6 +258,7 @@ static int build_table(BlockTable &t, const std::vector<long long> &items, int t
     CK(copy_in(stream, t.rep, rep.data(), rep.size() * sizeof(int)));
     CK(copy_in(stream, t.base, base.data(), base.size() * sizeof(long long)));
   }
+  CK(cudaStreamSynchronize(stream));
   return MCL_OK;
 }
 
@@ -609,6 +610,7 @@ int mcl_create(const mcl_model *model, const mcl_replica *replicas, int n_replic
     std::vector<uint8_t> p8(e->host_pt.begin(), e->host_pt.end());
     CKC(copy_in(e->stream, e->d_pt, p8.data(), p8.size()));
     CKC(copy_in(e->stream, e->d_nrm, ns.data(), ns.size() * sizeof(float)));
+    CKC(cudaStreamSynchronize(e->stream));
     for (int r = 0; r < n_replicas; r++) {
       const RepDesc &D = e->desc[r];
       long long nv = 0;
@@ -641,6 +643,7 @@ int mcl_create(const mcl_model *model, const mcl_replica *replicas, int n_replic
     }
     CKC(copy_in(e->stream, e->d_stage, aos.data(), aos.size() * sizeof(float)));
     for (int r = 0; r < n_replicas; r++) CKC(launch_unpack(e->ctx(), r, e->desc[r], e->d_stage));
+    CKC(cudaStreamSynchronize(e->stream));
   }
   if (schedule == MCL_SCHED_CHECKER2 && fused_supported(e)) {
     if ((rc = fused_create(e)) != MCL_OK) return cleanup_fail(rc);

@@ -17,8 +17,8 @@ namespace mcl {
 int fail(int code, const char *fmt, ...);
 int cuda_fail(cudaError_t err, const char *what);
 // Pageable host memory that a set-up prepared, to the device. On the stream whose kernels read it: the library's streams
-// do not wait for the default stream, whose copies from pageable memory may return before they end. The driver has
-// staged the source on return; whoever copies waits for the stream once, at the end of the set-up.
+// do not wait for the default stream, whose copies from pageable memory may return before they end. The caller waits for
+// the stream before the source goes: the driver may, but need not, have staged it on return.
 inline cudaError_t copy_in(cudaStream_t stream, void *d_dst, const void *src, size_t bytes) {
   return cudaMemcpyAsync(d_dst, src, bytes, cudaMemcpyHostToDevice, stream);
 }
